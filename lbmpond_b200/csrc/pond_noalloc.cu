@@ -7,8 +7,8 @@
 // loop, or a runtime that hands out device memory only through its own
 // allocator.  The context API allocates its double buffers and reduction
 // slots in pond_create; this entry point takes the caller's input and output
-// buffers and keeps its only scratch -- one partial-sum record per CTA of the
-// step kernel -- in a fixed array in this file's device memory.
+// buffers and keeps its only scratch -- an array of partial-sum records, each
+// shared by at most a few CTAs of the step kernel -- in a fixed array in this file's device memory.
 //
 // The scratch array is a file-scope __device__ variable: every GPU that
 // loads the library holds POND_NOALLOC_SCRATCH_BYTES of it until the process
@@ -28,8 +28,8 @@
 namespace pond {
 namespace noalloc {
 
-constexpr int kMaxBlocks = 65536;  // CTAs of the step kernel: 256^3 nodes at 32x4x2 per CTA
-constexpr size_t kScratchBytes = size_t(kMaxBlocks) * sizeof(d27::BlockPartial);
+constexpr int kMaxBlocks = 65536;  // largest grid accepted, in blocks of 32x4x2 nodes (256^3 nodes)
+constexpr size_t kScratchBytes = size_t(d27::PARTIALS) * sizeof(d27::BlockPartial);
 static_assert(kScratchBytes == POND_NOALLOC_SCRATCH_BYTES, "pond.h states the scratch size");
 
 static __device__ __align__(256) unsigned char g_partials[kScratchBytes];
@@ -38,9 +38,12 @@ constexpr int kMaxDevices = 64;
 static std::mutex g_setup_mutex;
 static void* g_partials_addr[kMaxDevices] = {};
 
-// Sum the per-CTA records in a fixed order (the result does not depend on
-// CTA scheduling) and write the step's diagnostics to the caller's buffer.
-__global__ void __launch_bounds__(256) reduce_partials_kernel(const d27::BlockPartial* part, int nblocks,
+// Sum the records in a fixed order and write the step's diagnostics to the
+// caller's buffer.  A record holds the sums of one or two CTAs up to 256^3
+// nodes in grids of three or more z planes, and two terms add to the same
+// value in either order, so the result does not depend on CTA scheduling
+// there; flatter grids near the size limit share a record among up to four.
+__global__ void __launch_bounds__(256) reduce_partials_kernel(const d27::BlockPartial* part, int nrec,
                                                               long long N, pond_diag* out) {
   __shared__ double sd[6][256];
   __shared__ unsigned long long su[2][256];
@@ -49,7 +52,7 @@ __global__ void __launch_bounds__(256) reduce_partials_kernel(const d27::BlockPa
   double v[6] = {0, 0, 0, 0, 0, 0};
   unsigned long long ni = 0, nc = 0;
   int mx = 0;
-  for (int b = t; b < nblocks; b += 256) {
+  for (int b = t; b < nrec; b += 256) {
     const d27::BlockPartial& p = part[b];
     v[0] += p.mass; v[1] += p.mom[0]; v[2] += p.mom[1]; v[3] += p.mom[2]; v[4] += p.enrg; v[5] += p.k;
     ni += p.niter_sum; nc += p.nonconv; mx = max(mx, p.niter_max);
@@ -145,15 +148,13 @@ extern "C" int pond_step_noalloc(const pond_params* p, const float* f_in, const 
   if (vst != POND_OK) return vst;
   for (int k = 0; k < 3; k++)
     if (p->bc[k] == POND_BC_INFLOW) return set_error(POND_ERR_UNSUPPORTED, "pond_step_noalloc has no inflow boundary");
-  const dim3 grd((unsigned)((p->Nx + d27::TX - 1) / d27::TX), (unsigned)((p->Ny + d27::TY - 1) / d27::TY),
-                 (unsigned)((p->Nz + d27::TZ - 1) / d27::TZ));
-  const long long nblocks = (long long)grd.x * grd.y * grd.z;
+  const long long nblocks = (long long)((p->Nx + 31) / 32) * ((p->Ny + 3) / 4) * ((p->Nz + 1) / 2);
   if (nblocks > noalloc::kMaxBlocks)
     return set_error(POND_ERR_ARG,
-                     "pond_step_noalloc: grid %lldx%lldx%lld needs %lld step CTAs; its fixed scratch holds %d "
-                     "(at most %d nodes, e.g. 256^3)",
+                     "pond_step_noalloc: grid %lldx%lldx%lld needs %lld blocks of 32x4x2 nodes; its fixed scratch "
+                     "serves %d (at most %d nodes, e.g. 256^3)",
                      (long long)p->Nx, (long long)p->Ny, (long long)p->Nz, nblocks, noalloc::kMaxBlocks,
-                     noalloc::kMaxBlocks * d27::THREADS);
+                     noalloc::kMaxBlocks * 256);
   if (noalloc::any_overlap(N, f_in, rho_in, g_in, f_out, rho_out, g_out))
     return set_error(POND_ERR_ARG, "pond_step_noalloc: an output buffer overlaps an input or another output");
   void* scratch = nullptr;
@@ -165,7 +166,7 @@ extern "C" int pond_step_noalloc(const pond_params* p, const float* f_in, const 
   a.f_out = f_out; a.rho_out = rho_out; a.g_out = g_out;
   a.guess = nullptr;
   a.niter_out = nullptr;
-  a.sums = reinterpret_cast<StepSums*>(scratch);  // the per-CTA partial records
+  a.sums = reinterpret_cast<StepSums*>(scratch);  // the partial records
   a.nx = (int)p->Nx; a.ny = (int)p->Ny; a.nz = (int)p->Nz;
   a.N = N;
   for (int k = 0; k < 3; k++) a.bc[k] = p->bc[k];
@@ -176,14 +177,20 @@ extern "C" int pond_step_noalloc(const pond_params* p, const float* f_in, const 
   const double PI = 3.14159265358979323846;
   a.kdx = 0.5 / (8 * PI * PI * PI) * (2 * PI / p->Nx) * (2 * PI / p->Ny) * (2 * PI / p->Nz);
   cudaStream_t s = (cudaStream_t)stream;
+  const dim3 grd((unsigned)((p->Nx + d27::TX - 1) / d27::TX), (unsigned)((p->Ny + d27::TY - 1) / d27::TY),
+                 (unsigned)((p->Nz + d27::TZ - 1) / d27::TZ));
   const dim3 blk(d27::TX, d27::TY, d27::TZ);
+  const long long ctas = (long long)grd.x * grd.y * grd.z;
+  const int nrec = (int)(ctas < d27::PARTIALS ? ctas : d27::PARTIALS);
+  cudaError_t e = cudaMemsetAsync(scratch, 0, (size_t)nrec * sizeof(d27::BlockPartial), s);
+  if (e != cudaSuccess) return cuda_fail(e, "pond_step_noalloc scratch reset");
   if (p->interp == POND_LAGR2) d27::pull_d3q27_tile_kernel<2, true><<<grd, blk, d27::SMEM_BYTES, s>>>(a);
   else if (p->interp == POND_LAGR3) d27::pull_d3q27_tile_kernel<3, true><<<grd, blk, d27::SMEM_BYTES, s>>>(a);
   else d27::pull_d3q27_tile_kernel<4, true><<<grd, blk, d27::SMEM_BYTES, s>>>(a);
-  cudaError_t e = cudaGetLastError();
+  e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "pond_step_noalloc step launch");
   noalloc::reduce_partials_kernel<<<1, 256, 0, s>>>(reinterpret_cast<const d27::BlockPartial*>(scratch),
-                                                      (int)nblocks, N, diag_out);
+                                                      nrec, N, diag_out);
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "pond_step_noalloc reduction launch");
   return POND_OK;

@@ -4,16 +4,18 @@
 // Same arithmetic as pull_point_kernel (steps.cu:356-588 LBMpull with
 // propagate<N>, N = 2, 3, 4), organised for the SM:
 //
-//  * a CTA owns a 32 x 4 x 2 tile of nodes and stages the tile plus a halo of
-//    2 nodes per side (36 x 8 x 6 nodes) once per step, node-major: a staged
+//  * a CTA owns an 8 x 4 x 4 tile of nodes and stages the tile plus a halo of
+//    2 nodes per side (12 x 8 x 8 nodes) once per step, node-major: a staged
 //    node's 27 populations are contiguous and 16-byte aligned (a 28-float
-//    stride, 189 KB), so a lane fetches a stencil node with seven 16-byte
+//    stride, 86 KB), so a lane fetches a stencil node with seven 16-byte
 //    loads, and the 28-word stride puts the eight lanes of every 16-byte load
-//    phase on distinct banks.  Each staging thread copies whole nodes and
-//    transfers them itself (no gauge planes in shared memory).  Boundary
-//    resolution (periodic wrap, clamp, mirror with population reversal), the
-//    reference's dropping of non-finite terms and the square root of T are
-//    applied while staging;
+//    phase on distinct banks.  Two CTAs share an SM (100 KB and 128 threads
+//    of 255 registers each): one stages while the other iterates, and neither
+//    waits for the other's slowest warp.  Each staging thread copies whole
+//    nodes and transfers them itself (no gauge planes in shared memory).
+//    Boundary resolution (periodic wrap, clamp, mirror with population
+//    reversal), the reference's dropping of non-finite terms and the square
+//    root of T are applied while staging;
 //  * after staging, each staged node's 27 populations are replaced by their
 //    transfer into a reference gauge shared by the CTA (the gauge of the
 //    tile's centre node).  The transfer of a source node into a target gauge
@@ -26,11 +28,24 @@
 //    reference-gauge populations one axis at a time (z per stencil node, y
 //    per stencil column, x per stencil row: 81 FMA each) instead of
 //    transforming every stencil node into the target gauge (243 FMA);
-//  * the fixed-point iteration is warp-synchronous: a warp iterates while any
-//    of its lanes is unconverged and walks the union of its lanes' stencil
-//    offsets, contracting every target class at every offset (a class a lane
-//    does not weight there has weight 0): straight-line code the scheduler
-//    interleaves;
+//  * the fixed-point iteration is warp-synchronous: a warp (an 8 x 4 patch of
+//    one z plane) iterates while any of its lanes is unconverged and walks the
+//    union of its lanes' stencil offsets, contracting every target class at
+//    every offset (a class a lane does not weight there has weight 0), except
+//    at the two ends of the usual z window (contract_tile);
+//  * the z and y contractions run as two-wide float32 multiply-adds on pairs
+//    of populations that the staged layout keeps in neighbouring registers
+//    (slot27): 45 instructions per stencil node instead of 81, for the same
+//    81 multiply-adds with the same roundings.
+//
+// What bounds it: the 128 B/clk of shared memory.  A stencil node costs 28
+// wavefronts per warp and 20-23 cycles of the SM's FMA pipes, so an iteration
+// of 125 nodes takes at least 3,500 cycles per warp of its SM: 20 ms of the
+// 30.0 ms that a 256^3 step of a half-uniform blast takes (46.1 ms in the
+// earlier form: 32 x 4 x 2 tiles, one CTA of 256 threads per SM, scalar
+// multiply-adds, rolled z offsets).  At 128^3, by ncu: shared-memory
+// wavefronts 70 % of peak, FMA pipe 52 % (the earlier form 40 %), issue slots
+// 52 %, 2.49 G warp instructions.
 //  * a lane whose departure points leave the +-2 halo (|u| + sqrt(T/TLat) >= 1
 //    along an axis) runs that iteration from global memory instead.
 #pragma once
@@ -39,9 +54,9 @@
 namespace pond {
 namespace d27 {
 
-constexpr int TX = 32, TY = 4, TZ = 2, H = 2;
+constexpr int TX = 8, TY = 4, TZ = 4, H = 2;
 constexpr int SX = TX + 2 * H, SY = TY + 2 * H, SZ = TZ + 2 * H;
-constexpr int SN = SX * SY * SZ;  // 1728 staged nodes
+constexpr int SN = SX * SY * SZ;  // 768 staged nodes
 constexpr int NS = 28;            // floats per staged node: its 27 R-gauge populations and a pad
 constexpr int THREADS = TX * TY * TZ;
 // staged nodes node-major (a node's populations contiguous, 16-byte aligned:
@@ -49,6 +64,16 @@ constexpr int THREADS = TX * TY * TZ;
 // lanes of each 16-byte load phase on distinct banks), then the iterate's
 // populations of every lane
 constexpr size_t SMEM_BYTES = size_t(NS) * SN * sizeof(float) + size_t(27) * THREADS * sizeof(float);
+static_assert(2 * (SMEM_BYTES + 2048) <= 233472, "two CTAs must fit in the 228 KB of an SM");
+
+// Slot of class (k1, k2, k3) in a staged node: the contractions along z and y
+// run on pairs of populations (two-wide float32 multiply-adds), so the
+// classes k1 = +, - of each (k2, k3) are neighbours (slots 0-17), the k1 = 0
+// classes k2 = +, - of each k3 (slots 18-23) and the three of k2 = 0 are last.
+__host__ __device__ constexpr int slot27(int k1, int k2, int k3) {
+  return k1 > 0 ? 2 * (3 * k2 + k3) + (k1 - 1) : k2 > 0 ? 18 + 2 * k3 + (k2 - 1) : 24 + k3;
+}
+__host__ __device__ constexpr int slot27(int t) { return slot27(t / 9, (t / 3) % 3, t % 3); }
 
 // reference population index of tensor class t = 9 cx + 3 cy + cz, for
 // lookups with run-time indices (consts.h:20-30 order)
@@ -178,9 +203,127 @@ template <int N> __device__ __forceinline__ float wpick(const float w[N], int ro
   return r;
 }
 
-// Per-CTA partial of the step sums, written instead of the atomic update
+// Two-wide float32 multiply-add with one factor shared by both halves.
+__device__ __forceinline__ float2 fma2(float g, float2 v, float2 o) { return __ffma2_rn(make_float2(g, g), v, o); }
+
+// One z offset of a stencil column: Z[k1,k2,i] += sum_k3 w_i Gz[i][k3] F[k1,k2,k3]
+// for the z-classes i in [I0, I1], i = 0 always (I0..I1 = 1..2: all three).
+// Zp[i][k2] holds the pair k1 = +, -; Zq[i] the pair k2 = +, - of k1 = 0; Zs[i] the rest.
+template <bool kPlus, bool kMinus>
+__device__ __forceinline__ void column_node(const float* node, const float Gz[3][3], const float w[3], float2 Zp[3][3],
+                                            float2 Zq[3], float Zs[3]) {
+  float4 v[7];
+  const float4* s4 = reinterpret_cast<const float4*>(node);
+#pragma unroll
+  for (int q = 0; q < 7; q++) v[q] = s4[q];
+  const auto pair = [&](int p) {  // slots 2p, 2p + 1
+    return (p & 1) ? make_float2(v[p >> 1].z, v[p >> 1].w) : make_float2(v[p >> 1].x, v[p >> 1].y);
+  };
+  const float last[3] = {v[6].x, v[6].y, v[6].z};
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    if ((i == 1 && !kPlus) || (i == 2 && !kMinus)) continue;
+#pragma unroll
+    for (int k3 = 0; k3 < 3; k3++) {
+      const float g = w[i] * Gz[i][k3];
+#pragma unroll
+      for (int k2 = 0; k2 < 3; k2++) Zp[i][k2] = fma2(g, pair(3 * k2 + k3), Zp[i][k2]);
+      Zq[i] = fma2(g, pair(9 + k3), Zq[i]);
+      Zs[i] = fmaf(g, last[k3], Zs[i]);
+    }
+  }
+}
+
+// The populations of one iterate from the staged, R-gauge nodes around `centre`
+// (the lane's node): acc[i1,i2,i3] = sum over the stencil offsets of the
+// interpolation weights times the transfer from the reference gauge to the
+// target, contracted along z per stencil node, y per column, x per row.  The
+// offsets walked are wl..wh per axis, the union over the warp's unconverged
+// lanes; a class a lane does not weight at an offset has weight 0 there.
+// `staggered` (warp-uniform): along z every lane's + class starts at wl and
+// its - class one later, wh = wl + N, as for |u_z| < c below one node per
+// step; then the first offset skips the - class and the last one the + class,
+// and the column is straight-line code.
+template <int N>
+__device__ __forceinline__ void contract_tile(const float* centre, int sx, int sxy, const int wl[3], const int wh[3],
+                                              bool staggered, const int ro[3][3], const float wt[3][3][N],
+                                              const float bq[3], float ainv, float acc[27]) {
+  float Gz[3][3];  // the z basis is used per stencil node; x and y are rebuilt per row and column
+  basis_rows(bq[2], ainv, Gz);
+  float wz[N + 1][3];  // z weights of the staggered window, by offset from wl
+#pragma unroll
+  for (int j = 0; j <= N; j++)
+#pragma unroll
+    for (int c = 0; c < 3; c++) wz[j][c] = wpick<N>(wt[2][c], ro[2][c], wl[2] + j);
+#pragma unroll 1
+  for (int ox = wl[0]; ox <= wh[0]; ox++) {
+    float2 Yp[3][3];
+    float Y0[3][3];
+#pragma unroll
+    for (int i2 = 0; i2 < 3; i2++)
+#pragma unroll
+      for (int i3 = 0; i3 < 3; i3++) { Yp[i2][i3] = make_float2(0.f, 0.f); Y0[i2][i3] = 0.f; }
+#pragma unroll 1
+    for (int oy = wl[1]; oy <= wh[1]; oy++) {
+      float2 Zp[3][3], Zq[3];
+      float Zs[3];
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+#pragma unroll
+        for (int k2 = 0; k2 < 3; k2++) Zp[i][k2] = make_float2(0.f, 0.f);
+        Zq[i] = make_float2(0.f, 0.f);
+        Zs[i] = 0.f;
+      }
+      const float* col = centre + (wl[2] * sxy + oy * sx + ox) * NS;
+      if (staggered) {
+        column_node<true, false>(col, Gz, wz[0], Zp, Zq, Zs);
+#pragma unroll
+        for (int j = 1; j < N; j++) column_node<true, true>(col + j * sxy * NS, Gz, wz[j], Zp, Zq, Zs);
+        column_node<false, true>(col + N * sxy * NS, Gz, wz[N], Zp, Zq, Zs);
+      } else {
+#pragma unroll 1
+        for (int oz = wl[2]; oz <= wh[2]; oz++) {
+          float w[3];
+#pragma unroll
+          for (int c = 0; c < 3; c++) w[c] = wpick<N>(wt[2][c], ro[2][c], oz);
+          column_node<true, true>(col + (oz - wl[2]) * sxy * NS, Gz, w, Zp, Zq, Zs);
+        }
+      }
+      float G[3][3];
+      basis_rows(bq[1], ainv, G);
+#pragma unroll
+      for (int i2 = 0; i2 < 3; i2++) {
+        const float w = wpick<N>(wt[1][i2], ro[1][i2], oy);
+        const float g0 = w * G[i2][0], g1 = w * G[i2][1], g2 = w * G[i2][2];
+#pragma unroll
+        for (int i3 = 0; i3 < 3; i3++) {
+          Yp[i2][i3] = fma2(g2, Zp[i3][2], fma2(g1, Zp[i3][1], fma2(g0, Zp[i3][0], Yp[i2][i3])));
+          Y0[i2][i3] = fmaf(g2, Zq[i3].y, fmaf(g1, Zq[i3].x, fmaf(g0, Zs[i3], Y0[i2][i3])));
+        }
+      }
+    }
+    float G[3][3];
+    basis_rows(bq[0], ainv, G);
+#pragma unroll
+    for (int i1 = 0; i1 < 3; i1++) {
+      const float w = wpick<N>(wt[0][i1], ro[0][i1], ox);
+      const float g0 = w * G[i1][0], g1 = w * G[i1][1], g2 = w * G[i1][2];
+#pragma unroll
+      for (int i2 = 0; i2 < 3; i2++)
+#pragma unroll
+        for (int i3 = 0; i3 < 3; i3++) {
+          float& o = acc[(i1 * 3 + i2) * 3 + i3];
+          o = fmaf(g2, Yp[i2][i3].y, fmaf(g1, Yp[i2][i3].x, fmaf(g0, Y0[i2][i3], o)));
+        }
+    }
+  }
+}
+
+// Partial record of the step sums, updated instead of the context's sums
 // when the kernel runs without a context (kPartials = true; a.sums then
-// points at an array of one BlockPartial per CTA).
+// points at an array of PARTIALS zeroed records, CTA b adding to record
+// b % PARTIALS).
+constexpr int PARTIALS = 65536;
 struct BlockPartial {
   double mass, mom[3], enrg, k;
   unsigned long long niter_sum, nonconv, work;
@@ -188,7 +331,7 @@ struct BlockPartial {
   int pad;
 };
 
-__device__ __forceinline__ void write_block_partial(NodeSums s, BlockPartial* out) {
+__device__ __forceinline__ void add_block_partial(NodeSums s, BlockPartial* out) {
   __shared__ double pd[6][THREADS / 32];
   __shared__ unsigned long long pu[3][THREADS / 32];
   __shared__ int pm[THREADS / 32];
@@ -217,12 +360,21 @@ __device__ __forceinline__ void write_block_partial(NodeSums s, BlockPartial* ou
       b.niter_sum += pu[0][w]; b.nonconv += pu[1][w]; b.work += pu[2][w];
       b.niter_max = max(b.niter_max, pm[w]);
     }
-    out[blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)] = b;
+    const unsigned long long cta =
+        blockIdx.x + (unsigned long long)gridDim.x * (blockIdx.y + (unsigned long long)gridDim.y * blockIdx.z);
+    BlockPartial* o = out + cta % PARTIALS;
+    atomicAdd(&o->mass, b.mass);
+    for (int q = 0; q < 3; q++) atomicAdd(&o->mom[q], b.mom[q]);
+    atomicAdd(&o->enrg, b.enrg);
+    atomicAdd(&o->k, b.k);
+    atomicAdd(&o->niter_sum, b.niter_sum);
+    if (b.nonconv) atomicAdd(&o->nonconv, b.nonconv);
+    atomicMax(&o->niter_max, b.niter_max);
   }
 }
 
 template <int N, bool kPartials = false>
-__global__ void __launch_bounds__(THREADS, 1) pull_d3q27_tile_kernel(StepArgs<float> a) {
+__global__ void __launch_bounds__(THREADS, 2) pull_d3q27_tile_kernel(StepArgs<float> a) {
   using L = Lattice<POND_D3Q27>;
   extern __shared__ __align__(16) float sm[];
   const int tid = threadIdx.x + TX * (threadIdx.y + TY * threadIdx.z);
@@ -259,6 +411,7 @@ __global__ void __launch_bounds__(THREADS, 1) pull_d3q27_tile_kernel(StepArgs<fl
   // comes straight from global memory (mirrored velocity components flip; a
   // node with a non-finite gauge contributes nothing, non-finite populations
   // count as 0)
+#pragma unroll 1
   for (int i = tid; i < SN; i += THREADS) {
     const int hx = i % SX, hy = (i / SX) % SY, hz = i / (SX * SY);
     bool rv[3];
@@ -272,10 +425,11 @@ __global__ void __launch_bounds__(THREADS, 1) pull_d3q27_tile_kernel(StepArgs<fl
       if (rv[0]) cx = rev3(cx);
       if (rv[1]) cy = rev3(cy);
       if (rv[2]) cz = rev3(cz);
-      cp_async4(&sm[i * NS + t], a.f_in + (long long)c_ref27[cx * 9 + cy * 3 + cz] * a.N + g);
+      cp_async4(&sm[i * NS + slot27(t)], a.f_in + (long long)c_ref27[cx * 9 + cy * 3 + cz] * a.N + g);
     }
   }
   cp_async_wait_all();
+#pragma unroll 1
   for (int i = tid; i < SN; i += THREADS) {
     const int hx = i % SX, hy = (i / SX) % SY, hz = i / (SX * SY);
     bool rv[3];
@@ -296,14 +450,17 @@ __global__ void __launch_bounds__(THREADS, 1) pull_d3q27_tile_kernel(StepArgs<fl
     ok = ok && fabsf(c) <= 3.0e38f;
     float v[27];
     {
+      float e[28];
       const float4* s4 = reinterpret_cast<const float4*>(sm + i * NS);
 #pragma unroll
       for (int q = 0; q < 7; q++) {
         const float4 w = s4[q];
-        const float e[4] = {w.x, w.y, w.z, w.w};
+        e[4 * q] = w.x; e[4 * q + 1] = w.y; e[4 * q + 2] = w.z; e[4 * q + 3] = w.w;
+      }
 #pragma unroll
-        for (int j = 0; j < 4; j++)
-          if (4 * q + j < 27) v[4 * q + j] = (ok && fabsf(e[j]) <= 3.402823466e38f) ? e[j] : 0.f;
+      for (int t = 0; t < 27; t++) {
+        const float w = e[slot27(t)];
+        v[t] = (ok && fabsf(w) <= 3.402823466e38f) ? w : 0.f;
       }
     }
     const float r = ok ? c * icref : 0.f;
@@ -312,10 +469,13 @@ __global__ void __launch_bounds__(THREADS, 1) pull_d3q27_tile_kernel(StepArgs<fl
     const float rq[3] = {r, r, r};
     node_to_ref(v, sq, rq);
     {
+      float e[28];
+      e[27] = 0.f;
+#pragma unroll
+      for (int t = 0; t < 27; t++) e[slot27(t)] = v[t];
       float4* s4 = reinterpret_cast<float4*>(sm + i * NS);
 #pragma unroll
-      for (int q = 0; q < 7; q++)
-        s4[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], 4 * q + 3 < 27 ? v[4 * q + 3] : 0.f);
+      for (int q = 0; q < 7; q++) s4[q] = make_float4(e[4 * q], e[4 * q + 1], e[4 * q + 2], e[4 * q + 3]);
     }
   }
   __syncthreads();
@@ -370,8 +530,6 @@ __global__ void __launch_bounds__(THREADS, 1) pull_d3q27_tile_kernel(StepArgs<fl
     float bq[3];
 #pragma unroll
     for (int ax = 0; ax < 3; ax++) bq[ax] = float((double(uref[ax]) - U[ax]) / C);
-    float Gz[3][3];  // the z basis is used per stencil node; x and y are rebuilt per row and column
-    basis_rows(bq[2], ainv, Gz);
     float acc[27];
 #pragma unroll
     for (int t = 0; t < 27; t++) acc[t] = 0.f;
@@ -384,52 +542,14 @@ __global__ void __launch_bounds__(THREADS, 1) pull_d3q27_tile_kernel(StepArgs<fl
         wl[ax] = __reduce_min_sync(0xffffffffu, done ? H : lo[ax]);
         wh[ax] = __reduce_max_sync(0xffffffffu, done ? -H : hi[ax]);
       }
-      // every target class at every offset (a class a lane does not weight
-      // there gets weight 0): branch-free contractions the scheduler can
-      // interleave, which measured faster than skipping the classes no lane
-      // of the warp weights (54.8 against 58.8 ms per 256^3 step)
-      const bool all3[3] = {true, true, true};
+      const bool staggered =
+          __all_sync(0xffffffffu, done || (ro[2][1] == wl[2] && ro[2][2] == wl[2] + 1 && ro[2][0] >= wl[2] &&
+                                           ro[2][0] <= wl[2] + 1)) && wh[2] == wl[2] + N;
       if (!done) {  // floating-point operations of the contractions below
         const unsigned long long ex = wh[0] - wl[0] + 1, ey = wh[1] - wl[1] + 1, ez = wh[2] - wl[2] + 1;
-        work += ex * ey * ez * (54ull * 3 + 9) + ex * ey * (54ull * 3 + 9) + ex * (54ull * 3 + 9);
+        work += ex * ey * (ez * 171 - (staggered ? 114 : 0)) + ex * ey * 171 + ex * 171;
       }
-      for (int ox = wl[0]; ox <= wh[0]; ox++) {
-        float wx[3];
-#pragma unroll
-        for (int c = 0; c < 3; c++) wx[c] = wpick<N>(wt[0][c], ro[0][c], ox);
-        float Yr[27];
-#pragma unroll
-        for (int t = 0; t < 27; t++) Yr[t] = 0.f;
-        for (int oy = wl[1]; oy <= wh[1]; oy++) {
-          float wy[3];
-#pragma unroll
-          for (int c = 0; c < 3; c++) wy[c] = wpick<N>(wt[1][c], ro[1][c], oy);
-          float Zc[27];
-#pragma unroll
-          for (int t = 0; t < 27; t++) Zc[t] = 0.f;
-#pragma unroll
-          for (int oz = -H; oz <= H; oz++) {
-            if (oz < wl[2] || oz > wh[2]) continue;
-            float wz[3];
-#pragma unroll
-            for (int c = 0; c < 3; c++) wz[c] = wpick<N>(wt[2][c], ro[2][c], oz);
-            const float4* s4 = reinterpret_cast<const float4*>(sm + (sbase + oz * SX * SY + oy * SX + ox) * NS);
-            float vv[28];
-#pragma unroll
-            for (int q = 0; q < 7; q++) {
-              const float4 w = s4[q];
-              vv[4 * q] = w.x; vv[4 * q + 1] = w.y; vv[4 * q + 2] = w.z; vv[4 * q + 3] = w.w;
-            }
-            contract_z(Gz, wz, all3, [&](int t) { return vv[t]; }, Zc);
-          }
-          float Gy[3][3];
-          basis_rows(bq[1], ainv, Gy);
-          contract_y(Gy, wy, all3, Zc, Yr);
-        }
-        float Gx[3][3];
-        basis_rows(bq[0], ainv, Gx);
-        contract_x(Gx, wx, all3, Yr, acc);
-      }
+      contract_tile<N>(sm + sbase * NS, SX, SX * SY, wl, wh, staggered, ro, wt, bq, ainv, acc);
     } else if (!done) {
       // departure points beyond the staged halo: this lane reads global memory
       // and transfers each stencil node into the reference gauge itself
@@ -437,6 +557,8 @@ __global__ void __launch_bounds__(THREADS, 1) pull_d3q27_tile_kernel(StepArgs<fl
                                ez = window_positions<N, 3>(ro[2]);
       work += ex * ey * ez * 171 + ex * ey * 171 + ex * 171;
       const bool all3[3] = {true, true, true};
+      float Gz[3][3];
+      basis_rows(bq[2], ainv, Gz);
       for (int ox = lo[0]; ox <= hi[0]; ox = window_next<N, 3>(ro[0], ox)) {
         bool rv[3] = {false, false, false};
         const int gx = resolve_axis(x + ox, a.nx, a.bc[0], rv[0]);
@@ -509,7 +631,7 @@ __global__ void __launch_bounds__(THREADS, 1) pull_d3q27_tile_kernel(StepArgs<fl
     finish_node<POND_D3Q27, float>(a, idx, f0, rho0, U, T, niter, conv, ns);
     ns.work = work;
   }
-  if constexpr (kPartials) write_block_partial(ns, reinterpret_cast<BlockPartial*>(a.sums));
+  if constexpr (kPartials) add_block_partial(ns, reinterpret_cast<BlockPartial*>(a.sums));
   else reduce_and_commit(ns, a.sums);
 }
 

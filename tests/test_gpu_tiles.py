@@ -1,0 +1,92 @@
+"""The staged tile kernels at the sizes and flows where their tiling can go
+wrong: grids of one node to one more than a tile along each axis, and gauges
+whose stencil windows take every route through the contraction.
+
+Tolerances: the float32 and float64 parity tolerances of test_gpu_parity.py
+(largest difference over the largest value of the oracle's field)."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from tests.states import perturbed_populations, smooth_state
+from tests.test_gpu_parity import TOL, _compare
+
+pytestmark = pytest.mark.gpu
+
+
+def _flow(shape, kind, seed):
+    """rho, g: subsonic (|u_z| < c, staggered z windows), drift (|u| > c inside the halo: the classes'
+    windows coincide), or sheared (lanes of one warp on both sides of a window change)."""
+    rho, g = smooth_state(shape, 3, seed=seed, modes=1, du=0.02)
+    if kind == "drift":
+        g[:3] *= 0.2
+        g[0] += 0.3
+        g[2] -= 0.55
+        g[3] *= 0.2  # c = 0.24
+    elif kind == "sheared":
+        n = np.arange(rho.size)
+        g[2] += np.where(n % 3 == 0, 0.5, -0.3)
+        g[1] += np.where(n % 5 == 0, -0.35, 0.2)
+        g[3] *= 0.3
+    return rho, g
+
+
+def _step_pair(orc, pond, lat, shape, interp, kind, precision="fp32", bc=(0, 0, 0), seed=3, max_iter=100):
+    rho, g = _flow(shape, kind, seed)
+    if precision == "fp32":  # the same starting state on both sides
+        rho, g = rho.astype(np.float32).astype(float), g.astype(np.float32).astype(float)
+    f = perturbed_populations(orc, lat, rho, g, seed=seed, eps=0.01)
+    if precision == "fp32":
+        f = f.astype(np.float32).astype(float)
+    with pond.Solver(lattice=lat, shape=shape, interp=interp, precision=precision, tau=0.8, bc=bc,
+                     max_iter=max_iter) as s:
+        s.set_state(rho, g, f=f)
+        s.step(1)
+        out = s.get_state()
+    ref, niter, nc = orc.step(orc.State(f, rho, g), lat, shape, interp=interp, tau=0.8, bc=bc, max_iter=max_iter)
+    return out, ref, nc
+
+
+@pytest.mark.parametrize("interp", [2, 3, 4])
+@pytest.mark.parametrize("kind", ["subsonic", "drift"])
+@pytest.mark.parametrize("shape", [(1, 1, 1), (8, 4, 4), (9, 5, 5), (7, 3, 9), (17, 8, 3)])
+def test_d3q27_tile_edges(orc, pond, shape, kind, interp):
+    out, ref, nc = _step_pair(orc, pond, 1, shape, interp, kind)
+    assert nc == 0
+    _compare(out, ref, TOL["fp32"], f"{shape} {kind} {interp}")
+
+
+@pytest.mark.parametrize("interp", [2, 3, 4])
+def test_d3q27_windows_change_within_a_warp(orc, pond, interp):
+    """One iteration on a state whose neighbouring nodes differ in the windows they read.  The iterate's
+    populations are compared; its gauge is a ratio of them, and this state's densities cross zero."""
+    (f, rho, _), ref, _ = _step_pair(orc, pond, 1, (16, 8, 8), interp, "sheared", max_iter=1)
+    assert np.abs(f - ref.f).max() <= TOL["fp32"] * np.abs(ref.f).max()
+    assert np.abs(rho - ref.rho).max() <= TOL["fp32"] * np.abs(ref.rho).max()
+
+
+def test_noalloc_records_shared_by_ctas(pond):
+    """A grid of more CTAs than partial-sum records: the step's sums against the context's."""
+    import torch
+    from lbmpond_b200 import _lib
+    from tests.test_zz_no_alloc import _bind
+    L = _lib.load()
+    shape = (256, 256, 130)
+    N = int(np.prod(shape))
+    with pond.Solver(lattice="D3Q27", shape=shape, interp=3, precision="fp32", tau=0.8) as s:
+        s.init("tgv", 0.05, 0.1, 1.0, 5.0 / 3.0)
+        ptr = s.device_state()
+        out = [torch.empty(n, dtype=torch.float32, device="cuda") for n in (27 * N, N, 4 * N)]
+        diag = torch.zeros(ctypes.sizeof(_lib.PondDiag), dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+        p = s.get_params()
+        st = _bind(L)(ctypes.byref(p), *ptr, *(t.data_ptr() for t in out), diag.data_ptr(),
+                      torch.cuda.current_stream().cuda_stream)
+        assert st == 0, L.pond_last_error_string().decode()
+        torch.cuda.synchronize()
+        s.step(1)
+        want = s.diagnostics()
+    d = _lib.PondDiag.from_buffer_copy(bytes(diag.cpu().numpy()))
+    assert abs(d.mass - want["mass"]) <= 1e-12 * want["mass"] and abs(d.enrg - want["enrg"]) <= 1e-12 * want["enrg"]
+    assert d.niter_sum == want["niter_sum"] and d.niter_max == want["niter_max"]
