@@ -11,6 +11,7 @@
 #include "pond_step_1d_mesh.cuh"
 #include "pond_step_d3q27_energy.cuh"
 #include "pond_step_d3q27_energy_tile.cuh"
+#include "pond_step_d3q125_rows.cuh"
 #include "pond_step_d3q125_tile.cuh"
 #include "pond_step_d3q27.cuh"
 #include "pond_step_point.cuh"
@@ -355,16 +356,24 @@ template <typename R> static int launch_typed(pond_ctx* c, const void* const* in
         default: return set_error(POND_ERR_UNSUPPORTED, "scheme");
       }
       break;
-    case POND_D3Q125: {  // staged tile, reference-gauge transfer (float64: one CTA per SM)
-      const size_t smem = sizeof(d125t::SmemT<false, R>);
-      e = cudaFuncSetAttribute(d125t::pull_d3q125_tile_kernel<false, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)smem);
-      if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute");
-      const dim3 grd((a.nx + d125t::T - 1) / d125t::T, (a.ny + d125t::T - 1) / d125t::T,
-                     (a.nz + d125t::T - 1) / d125t::T);
-      d125t::pull_d3q125_tile_kernel<false, R><<<grd, d125t::THREADS, smem, s>>>(a);
+    case POND_D3Q125:  // staged tile, reference-gauge transfer
+      if constexpr (std::is_same<R, float>::value) {
+        const size_t smem = sizeof(d125r::Smem);
+        e = cudaFuncSetAttribute(d125r::pull_d3q125_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute");
+        const dim3 grd((a.nx + d125r::TX - 1) / d125r::TX, (a.ny + d125r::TY - 1) / d125r::TY,
+                       (a.nz + d125r::TZ - 1) / d125r::TZ);
+        d125r::pull_d3q125_rows_kernel<<<grd, d125r::THREADS, smem, s>>>(a);
+      } else {  // float64: a warp per node, one CTA per SM
+        const size_t smem = sizeof(d125t::SmemT<false, R>);
+        e = cudaFuncSetAttribute(d125t::pull_d3q125_tile_kernel<false, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)smem);
+        if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute");
+        const dim3 grd((a.nx + d125t::T - 1) / d125t::T, (a.ny + d125t::T - 1) / d125t::T,
+                       (a.nz + d125t::T - 1) / d125t::T);
+        d125t::pull_d3q125_tile_kernel<false, R><<<grd, d125t::THREADS, smem, s>>>(a);
+      }
       break;
-    }
     default: return set_error(POND_ERR_UNSUPPORTED, "lattice");
   }
   e = cudaGetLastError();

@@ -17,13 +17,16 @@ pytestmark = pytest.mark.gpu
 
 def _flow(shape, kind, seed):
     """rho, g: subsonic (|u_z| < c, staggered z windows), drift (|u| > c inside the halo: the classes'
-    windows coincide), or sheared (lanes of one warp on both sides of a window change)."""
+    windows coincide), crosswind (off-centre WENO windows), or sheared (lanes of one warp on both sides of a window change)."""
     rho, g = smooth_state(shape, 3, seed=seed, modes=1, du=0.02)
     if kind == "drift":
         g[:3] *= 0.2
         g[0] += 0.3
         g[2] -= 0.55
         g[3] *= 0.2  # c = 0.24
+    elif kind == "crosswind":
+        g[2] += 0.3  # moves some classes' z windows by a node
+        g[1] -= 0.25
     elif kind == "sheared":
         n = np.arange(rho.size)
         g[2] += np.where(n % 3 == 0, 0.5, -0.3)
@@ -64,6 +67,15 @@ def test_d3q27_windows_change_within_a_warp(orc, pond, interp):
     (f, rho, _), ref, _ = _step_pair(orc, pond, 1, (16, 8, 8), interp, "sheared", max_iter=1)
     assert np.abs(f - ref.f).max() <= TOL["fp32"] * np.abs(ref.f).max()
     assert np.abs(rho - ref.rho).max() <= TOL["fp32"] * np.abs(ref.rho).max()
+
+
+@pytest.mark.parametrize("bc", [(0, 0, 0), (2, 1, 0)])
+@pytest.mark.parametrize("shape", [(1, 1, 1), (6, 4, 4), (7, 5, 3), (13, 2, 9)])
+def test_d3q125_row_edges(orc, pond, shape, bc):
+    """Fixed-origin quadratic: six nodes of a row per warp, 6 x 4 x 4 tiles."""
+    out, ref, nc = _step_pair(orc, pond, 2, shape, 6, "subsonic", bc=bc)
+    assert nc == 0
+    _compare(out, ref, TOL["fp32"], f"{shape} {bc}")
 
 
 def test_noalloc_records_shared_by_ctas(pond):
