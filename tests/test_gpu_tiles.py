@@ -78,6 +78,15 @@ def test_d3q125_row_edges(orc, pond, shape, bc):
     _compare(out, ref, TOL["fp32"], f"{shape} {bc}")
 
 
+@pytest.mark.parametrize("kind", ["subsonic", "crosswind"])
+@pytest.mark.parametrize("shape", [(4, 2, 2), (5, 3, 3), (3, 5, 1)])
+def test_d3q125_weno_tile_edges(orc, pond, shape, kind):
+    """Centred WENO5: 4 x 2 x 2 tiles, the usual z windows and others."""
+    out, ref, nc = _step_pair(orc, pond, 2, shape, 11, kind)
+    assert nc == 0
+    _compare(out, ref, TOL["fp32"], f"{shape} {kind}")
+
+
 def test_noalloc_records_shared_by_ctas(pond):
     """A grid of more CTAs than partial-sum records: the step's sums against the context's."""
     import torch
