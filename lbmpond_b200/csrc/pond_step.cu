@@ -10,6 +10,7 @@
 #include "pond_step_1d_energy.cuh"
 #include "pond_step_1d_mesh.cuh"
 #include "pond_step_d3q27_energy.cuh"
+#include "pond_step_d3q27_f64.cuh"
 #include "pond_step_d3q27_energy_tile.cuh"
 #include "pond_step_d3q125_rows.cuh"
 #include "pond_step_d3q125_tile.cuh"
@@ -347,14 +348,20 @@ template <typename R> static int launch_typed(pond_ctx* c, const void* const* in
           kern<<<grd, blk, d27::SMEM_BYTES, s>>>(a);
           break;
         }
+      } else if (c->p.interp >= POND_LAGR2 && c->p.interp <= POND_LAGR4) {
+        const dim3 grd((a.nx + d27d::TX - 1) / d27d::TX, (a.ny + d27d::TY - 1) / d27d::TY,
+                       (a.nz + d27d::TZ - 1) / d27d::TZ);
+        void (*kern)(StepArgs<double>) = c->p.interp == POND_LAGR2   ? d27d::pull_d3q27_f64_kernel<2>
+                                         : c->p.interp == POND_LAGR3 ? d27d::pull_d3q27_f64_kernel<3>
+                                                                     : d27d::pull_d3q27_f64_kernel<4>;
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(d27d::Smem));
+        if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute");
+        kern<<<grd, d27d::THREADS, sizeof(d27d::Smem), s>>>(a);
+        break;
       }
-      switch (c->p.interp) {
-        case POND_LAGR2: launch_point<POND_D3Q27, 2, R>(a, s); break;
-        case POND_LAGR3: launch_point<POND_D3Q27, 3, R>(a, s); break;
-        case POND_LAGR4: launch_point<POND_D3Q27, 4, R>(a, s); break;
-        case POND_LAGR5: launch_point<POND_D3Q27, 5, R>(a, s); break;
-        default: return set_error(POND_ERR_UNSUPPORTED, "scheme");
-      }
+      // order 5 (its windows reach three nodes out, past the tiles' halo)
+      if (c->p.interp != POND_LAGR5) return set_error(POND_ERR_UNSUPPORTED, "scheme");
+      launch_point<POND_D3Q27, 5, R>(a, s);
       break;
     case POND_D3Q125:  // staged tile, reference-gauge transfer
       if constexpr (std::is_same<R, float>::value) {

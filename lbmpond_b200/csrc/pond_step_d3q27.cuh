@@ -95,14 +95,14 @@ __device__ __forceinline__ int rev3(int c) { return c == 0 ? 0 : 3 - c; }
 // L_+ = y (y + 1) / 2, L_- = y (y - 1) / 2.  B is the one-axis gauge
 // transfer (structs.cuh:343-551) from a gauge (u, c) to (U, C) for
 // s = (u - U) / C, r = c / C.
-__device__ __forceinline__ void basis_rows(float s, float r, float B[3][3]) {
-  const float y[3] = {s, s + r, s - r};
+template <typename R> __device__ __forceinline__ void basis_rows(R s, R r, R B[3][3]) {
+  const R y[3] = {s, s + r, s - r};
 #pragma unroll
   for (int b = 0; b < 3; b++) {
-    const float yb = y[b], h = 0.5f * yb;
-    B[0][b] = fmaf(-yb, yb, 1.f);
-    B[1][b] = fmaf(h, yb, h);
-    B[2][b] = fmaf(h, yb, -h);
+    const R yb = y[b], h = R(0.5) * yb;
+    B[0][b] = fma(-yb, yb, R(1));
+    B[1][b] = fma(h, yb, h);
+    B[2][b] = fma(h, yb, -h);
   }
 }
 
@@ -111,20 +111,20 @@ __device__ __forceinline__ void basis_rows(float s, float r, float B[3][3]) {
 // s = (u - u_ref) / c_ref, r = c / c_ref.  A transfer into the target gauge
 // then equals the transfer of the result from (u_ref, c_ref) to the target,
 // because the basis reproduces every quadratic in the particle velocity.
-__device__ __forceinline__ void node_to_ref(float v[27], const float s[3], const float r[3]) {
+template <typename R> __device__ __forceinline__ void node_to_ref(R v[27], const R s[3], const R r[3]) {
 #pragma unroll
   for (int ax = 0; ax < 3; ax++) {
-    float B[3][3];
+    R B[3][3];
     basis_rows(s[ax], r[ax], B);
     const int st = ax == 0 ? 9 : ax == 1 ? 3 : 1;
 #pragma unroll
     for (int o = 0; o < 9; o++) {
       // the two other axes' indices
       const int base = ax == 0 ? o : ax == 1 ? (o / 3) * 9 + (o % 3) : o * 3;
-      const float f0 = v[base], fp = v[base + st], fm = v[base + 2 * st];
+      const R f0 = v[base], fp = v[base + st], fm = v[base + 2 * st];
 #pragma unroll
       for (int i = 0; i < 3; i++) {
-        const float o3 = fmaf(B[i][2], fm, fmaf(B[i][1], fp, B[i][0] * f0));
+        const R o3 = fma(B[i][2], fm, fma(B[i][1], fp, B[i][0] * f0));
         if (i == 0) v[base] = o3; else if (i == 1) v[base + st] = o3; else v[base + 2 * st] = o3;
       }
     }
@@ -195,9 +195,9 @@ __device__ __forceinline__ void contract_x(const float Gx[3][3], const float wx[
 }
 
 // interpolation weight of relative offset o for a window starting at ro
-template <int N> __device__ __forceinline__ float wpick(const float w[N], int ro, int o) {
+template <int N, typename R> __device__ __forceinline__ R wpick(const R w[N], int ro, int o) {
   const int j = o - ro;
-  float r = 0.f;
+  R r = R(0);
 #pragma unroll
   for (int k = 0; k < N; k++) r = (j == k) ? w[k] : r;
   return r;

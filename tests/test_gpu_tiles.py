@@ -17,7 +17,7 @@ pytestmark = pytest.mark.gpu
 
 def _flow(shape, kind, seed):
     """rho, g: subsonic (|u_z| < c, staggered z windows), drift (|u| > c inside the halo: the classes'
-    windows coincide), crosswind (off-centre WENO windows), or sheared (lanes of one warp on both sides of a window change)."""
+    windows coincide), crosswind (off-centre WENO windows), fast (beyond the halos), or sheared (lanes of one warp on both sides of a window change)."""
     rho, g = smooth_state(shape, 3, seed=seed, modes=1, du=0.02)
     if kind == "drift":
         g[:3] *= 0.2
@@ -27,6 +27,9 @@ def _flow(shape, kind, seed):
     elif kind == "crosswind":
         g[2] += 0.3  # moves some classes' z windows by a node
         g[1] -= 0.25
+    elif kind == "fast":  # departure points beyond every staged halo
+        g[0] += 1.6
+        g[2] -= 1.1
     elif kind == "sheared":
         n = np.arange(rho.size)
         g[2] += np.where(n % 3 == 0, 0.5, -0.3)
@@ -58,6 +61,16 @@ def test_d3q27_tile_edges(orc, pond, shape, kind, interp):
     out, ref, nc = _step_pair(orc, pond, 1, shape, interp, kind)
     assert nc == 0
     _compare(out, ref, TOL["fp32"], f"{shape} {kind} {interp}")
+
+
+@pytest.mark.parametrize("interp", [2, 3, 4])
+@pytest.mark.parametrize("kind,bc", [("subsonic", (2, 1, 0)), ("drift", (0, 0, 0)), ("fast", (0, 2, 1))])
+@pytest.mark.parametrize("shape", [(1, 1, 1), (10, 4, 2), (11, 5, 3), (9, 3, 5), (21, 2, 4)])
+def test_d3q27_float64_tile_edges(orc, pond, shape, kind, bc, interp):
+    """Ten nodes of a row per warp, 10 x 4 x 2 tiles; both routes of the iteration."""
+    out, ref, nc = _step_pair(orc, pond, 1, shape, interp, kind, precision="fp64", bc=bc)
+    assert nc == 0
+    _compare(out, ref, TOL["fp64"], f"{shape} {kind} {interp}")
 
 
 @pytest.mark.parametrize("interp", [2, 3, 4])
