@@ -186,6 +186,8 @@ template <typename R> struct StepArgs {
   const double* pos = nullptr;    // [N]
   // state of the inflow ghost node of POND_BC_INFLOW axes: rho, u_x, u_y, u_z, T
   double inflow[5] = {1, 0, 0, 0, 1};
+  // float64 D3Q27 tiles: 1 = left to the one-thread-per-node kernel, or null
+  uint8_t* tile_flags = nullptr;
 };
 
 }  // namespace pond

@@ -20,6 +20,7 @@ struct pond_ctx {
   pond::StepSums* d_sums = nullptr;
   pond::StepSums* h_sums = nullptr;  // pinned
   bool have_sums = false;
+  uint8_t* tile_flags = nullptr;  // float64 D3Q27, Lagrange 2-4: one per tile of the step
   int* niter = nullptr;
   bool keep_niter = false;
   float* guess = nullptr;  // [4][N] predicted starting gauge (learned path)

@@ -36,6 +36,14 @@ int ctx_alloc(pond_ctx* c) {
                        (size_t)(c->Q * (c->p.ddf ? 2 : 1) + 5) * N * c->elem);
     }
   }
+  if (c->p.lattice == POND_D3Q27 && c->elem == 8 && !c->p.ddf && c->p.interp <= POND_LAGR4) {
+    const size_t tiles = (size_t)((c->p.Nx + F64_TX - 1) / F64_TX) * (size_t)((c->p.Ny + F64_TY - 1) / F64_TY) *
+                         (size_t)((c->p.Nz + F64_TZ - 1) / F64_TZ);
+    if (cudaMalloc(&c->tile_flags, tiles) != cudaSuccess) {
+      cudaGetLastError();
+      return set_error(POND_ERR_NOMEM, "tile flags");
+    }
+  }
   if (cudaMalloc(&c->d_sums, sizeof(StepSums)) != cudaSuccess) {
     cudaGetLastError();
     return set_error(POND_ERR_NOMEM, "step sums");
@@ -54,6 +62,7 @@ void ctx_free(pond_ctx* c) {
     c->f[b] = c->rho[b] = c->g[b] = c->h[b] = nullptr;
   }
   cudaFree(c->d_sums); c->d_sums = nullptr;
+  cudaFree(c->tile_flags); c->tile_flags = nullptr;
   cudaFree(c->niter); c->niter = nullptr;
   cudaFree(c->guess); c->guess = nullptr;
   cudaFree(c->g_hist); c->g_hist = nullptr;
@@ -356,7 +365,12 @@ template <typename R> static int launch_typed(pond_ctx* c, const void* const* in
                                                                      : d27d::pull_d3q27_f64_kernel<4>;
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(d27d::Smem));
         if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute");
+        a.tile_flags = c->tile_flags;
         kern<<<grd, d27d::THREADS, sizeof(d27d::Smem), s>>>(a);
+        // the tiles it left
+        if (c->p.interp == POND_LAGR2) launch_point<POND_D3Q27, 2, R>(a, s);
+        else if (c->p.interp == POND_LAGR3) launch_point<POND_D3Q27, 3, R>(a, s);
+        else launch_point<POND_D3Q27, 4, R>(a, s);
         break;
       }
       // order 5 (its windows reach three nodes out, past the tiles' halo)

@@ -21,6 +21,13 @@
 //  * a warp with a node whose windows leave the halo runs that iteration from
 //    global memory: lane 3n + j transforms each stencil node into the target's
 //    z-class j directly, as the one-thread-per-node kernel does for all three.
+//    That takes 2.5-3.5 times the time of the one-thread-per-node kernel (32^3
+//    at c = 1.2: 10.6 against 4.1 ms, 10 nodes per warp instead of 32 and three
+//    loads of each), so it serves nodes that get there while iterating; a tile
+//    with a node that starts near the edge of the halo (|u| + c >= 0.98 on an
+//    axis for N = 4) is flagged and left to that kernel, which follows every
+//    launch and returns at once where nothing is flagged (32^3 at c = 0.95 and
+//    |u| up to 0.06: 4.0 ms with a quarter of the rows as the line, against 2.2).
 //
 // What bounds it: the float64 pipe (64 multiply-adds per clock and SM: 4,185 per
 // lane and iteration at N = 4 are 2,090 cycles of the SM) and shared-memory
@@ -34,7 +41,7 @@
 namespace pond {
 namespace d27d {
 
-constexpr int TX = 10, TY = 4, TZ = 2, H = 2;
+constexpr int TX = F64_TX, TY = F64_TY, TZ = F64_TZ, H = 2;
 constexpr int SX = TX + 2 * H, SY = TY + 2 * H, SZ = TZ + 2 * H;
 constexpr int SN = SX * SY * SZ;  // 672 staged nodes
 constexpr int NS = 30;            // doubles per staged node: slices k1 of nine, 10 apart
@@ -80,6 +87,29 @@ template <int N> __global__ void __launch_bounds__(THREADS, 1) pull_d3q27_f64_ke
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY, z0 = blockIdx.z * TZ;
   constexpr double kMax = 1.7976931348623157e308;
+
+  // ---- a tile with a node that starts at the edge of the halo or beyond is left to
+  //      the one-thread-per-node kernel launched after this one
+  {
+    const int n = lane % TX, x = x0 + n, y = y0 + warp % TY, z = z0 + warp / TY;
+    const bool here = x < a.nx && y < a.ny && z < a.nz;
+    bool far = false;
+    if (here && lane < TX) {
+      const long long g = x + (long long)a.nx * (y + (long long)a.ny * z);
+      const double c = a.guess ? sqrt(double(a.guess[3 * a.N + g]) * (1.0 / L::TLat))
+                               : sqrt(a.g_in[3 * a.N + g] * (1.0 / L::TLat));
+#pragma unroll
+      for (int ax = 0; ax < 3; ax++) {
+        const double u = fabs(a.guess ? double(a.guess[ax * a.N + g]) : a.g_in[ax * a.N + g]);
+        // the largest |v| whose window stays within two nodes, less what an iterate may add
+        far = far || u + c >= 0.98 * (N == 4 ? 1.0 : N == 2 ? 2.0 : ax == 0 ? 1.5 : 1.0);
+      }
+    }
+    const bool leave = __syncthreads_or(far);
+    if (tid == 0)
+      a.tile_flags[blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z)] = leave;
+    if (leave) return;
+  }
 
   // ---- reference gauge of the CTA: the gauge of the tile's centre node
   //      ((0, 1) if it is not finite or its c is 0)

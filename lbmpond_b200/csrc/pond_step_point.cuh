@@ -325,8 +325,13 @@ __device__ __forceinline__ void finish_node(const StepArgs<R>& a, long long idx,
   ns.niter = niter; ns.nonconv = conv ? 0 : 1; ns.nmax = niter;
 }
 
+// Nodes per axis of the tiles that StepArgs::tile_flags describes
+// (pond_step_d3q27_f64.cuh).
+constexpr int F64_TX = 10, F64_TY = 4, F64_TZ = 2;
+
 // One pull step, one thread per node, D1Q5 (1D lines) or D3Q27, Lagrange
-// interpolation of order N (steps.cu:986 propagate<N>).
+// interpolation of order N (steps.cu:986 propagate<N>).  With tile_flags, only
+// the nodes of flagged tiles.
 template <int LAT, int N, typename R>
 __global__ void __launch_bounds__(128) pull_point_kernel(StepArgs<R> a) {
   using L = Lattice<LAT>;
@@ -334,7 +339,14 @@ __global__ void __launch_bounds__(128) pull_point_kernel(StepArgs<R> a) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   const int z = blockIdx.z * blockDim.z + threadIdx.z;
-  const bool active = x < a.nx && y < a.ny && z < a.nz;
+  bool active = x < a.nx && y < a.ny && z < a.nz;
+  if constexpr (LAT == POND_D3Q27 && sizeof(R) == 8) {
+    if (a.tile_flags) {
+      const int tx = (a.nx + F64_TX - 1) / F64_TX, ty = (a.ny + F64_TY - 1) / F64_TY;
+      active = active && a.tile_flags[x / F64_TX + (long long)tx * (y / F64_TY + (long long)ty * (z / F64_TZ))] != 0;
+      if (!__syncthreads_or(active)) return;
+    }
+  }
   NodeSums ns = {0, 0, 0, 0, 0, 0, 0ull, 0ull, 0ull, 0};
   if (active) {
     const long long idx = x + (long long)a.nx * (y + (long long)a.ny * z);

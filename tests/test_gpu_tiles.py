@@ -73,6 +73,26 @@ def test_d3q27_float64_tile_edges(orc, pond, shape, kind, bc, interp):
     _compare(out, ref, TOL["fp64"], f"{shape} {kind} {interp}")
 
 
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("interp", [3, 4])
+def test_d3q27_iterates_leave_the_halo(orc, pond, interp, precision):
+    """Gauges that start inside the halo and iterate past it: the populations carry more momentum."""
+    shape = (13, 6, 5)
+    rho, g = smooth_state(shape, 3, seed=9, modes=1, T0=0.05, du=0.01, dT=0.002)
+    g[1] += 0.55  # |u_y| + c = 0.95 at the start
+    xi = pond.lattice_tables(1)[0]
+    f = perturbed_populations(orc, 1, rho, g, seed=9, eps=0.01) * (1 + 1.2 * xi[:, 1:2])
+    if precision == "fp32":
+        rho, g, f = (a.astype(np.float32).astype(float) for a in (rho, g, f))
+    with pond.Solver(lattice=1, shape=shape, interp=interp, precision=precision, tau=0.8) as s:
+        s.set_state(rho, g, f=f)
+        s.step(1)
+        out = s.get_state()
+    ref, niter, nc = orc.step(orc.State(f, rho, g), 1, shape, interp=interp, tau=0.8)
+    assert nc == 0 and (np.abs(ref.g[1]) + np.sqrt(3 * ref.g[3])).max() > 1.0
+    _compare(out, ref, TOL[precision], f"{interp} {precision}")
+
+
 @pytest.mark.parametrize("interp", [2, 3, 4])
 def test_d3q27_windows_change_within_a_warp(orc, pond, interp):
     """One iteration on a state whose neighbouring nodes differ in the windows they read.  The iterate's
