@@ -555,7 +555,10 @@ int pond_step(pond_ctx* c, int nsteps) {
   cudaError_t e = cudaEventRecord(c->ev0, c->stream);
   if (e != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
   for (int s = 0; s < nsteps; s++) {
+    // only the sums of the last step are kept, unless each step's are read
+    c->reset_sums = s == nsteps - 1 || c->strict || c->dt_adapt;
     int st = launch_step(c);
+    c->reset_sums = true;
     if (st != POND_OK) return st;
     c->cur = 1 - c->cur;  // LBMParamsHost::swapLS (structs.cuh:148)
     c->istep++;

@@ -20,6 +20,7 @@ struct pond_ctx {
   pond::StepSums* d_sums = nullptr;
   pond::StepSums* h_sums = nullptr;  // pinned
   bool have_sums = false;
+  bool reset_sums = true;  // the next step starts its sums from zero; the steps before the last of a run need not
   uint8_t* tile_flags = nullptr;  // float64 D3Q27, Lagrange 2-4: one per tile of the step
   int* niter = nullptr;
   bool keep_niter = false;

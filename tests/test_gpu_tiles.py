@@ -120,6 +120,30 @@ def test_d3q125_weno_tile_edges(orc, pond, shape, kind):
     _compare(out, ref, TOL["fp32"], f"{shape} {kind}")
 
 
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("interp", [2, 3, 4, 5, 7, 8])
+@pytest.mark.parametrize("nx,kind,bc", [(3, "subsonic", 1), (8, "subsonic", 2), (9, "fast", 0), (37, "fast", 1),
+                                        (4096, "subsonic", 0), (4097, "subsonic", 0)])
+def test_d1q5_warp_and_thread_per_node(orc, pond, nx, kind, bc, interp, precision):
+    """One node per warp up to 4096 nodes, one per thread above; windows of |v| above and below one node."""
+    rho, g = smooth_state((nx, 1, 1), 1, seed=nx, modes=1, T0=0.02, du=0.02, dT=0.002)
+    if kind == "fast":
+        g[0] += 1.4
+    f = perturbed_populations(orc, 0, rho, g, seed=nx, eps=0.01)
+    if precision == "fp32":
+        rho, g, f = (a.astype(np.float32).astype(float) for a in (rho, g, f))
+    with pond.Solver(lattice=0, shape=(nx, 1, 1), interp=interp, precision=precision, tau=0.8, bc=(bc, 0, 0)) as s:
+        s.set_state(rho, g, f=f)
+        s.step(1)
+        out, d = s.get_state(), s.diagnostics()
+    ref, niter, nc = orc.step(orc.State(f, rho, g), 0, (nx, 1, 1), interp=interp, tau=0.8, bc=(bc, 0, 0))
+    assert nc == 0 and d["nonconverged"] == 0
+    _compare(out, ref, TOL[precision], f"{nx} {kind} {interp}")
+    if precision == "fp64":
+        assert d["niter_max"] == int(niter.max())
+        assert abs(d["mass"] - ref.rho.sum()) <= 1e-9 * ref.rho.sum()
+
+
 def test_noalloc_records_shared_by_ctas(pond):
     """A grid of more CTAs than partial-sum records: the step's sums against the context's."""
     import torch
