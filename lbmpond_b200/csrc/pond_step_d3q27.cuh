@@ -33,6 +33,11 @@
 //    union of its lanes' stencil offsets, contracting every target class at
 //    every offset (a class a lane does not weight there has weight 0), except
 //    at the two ends of the usual z window (contract_tile);
+//  * once only a few lanes of a warp still iterate, the warp serves their nodes
+//    one at a time, a stencil column per lane: a node that runs to the
+//    iteration cap then takes 2 us per iteration instead of 11 to 20, which is
+//    what the end of a step waited for (two nodes of a 128^3 vortex at the cap:
+//    3.87 -> 3.38 ms; two steps with energy populations at 64^3: 4.39 -> 2.46 ms);
 //  * the z and y contractions run as two-wide float32 multiply-adds on pairs
 //    of populations that the staged layout keeps in neighbouring registers
 //    (slot27): 45 instructions per stencil node instead of 81, for the same
@@ -63,7 +68,8 @@ constexpr int THREADS = TX * TY * TZ;
 // seven 16-byte loads per stencil node; the 28-word stride keeps the eight
 // lanes of each 16-byte load phase on distinct banks), then the iterate's
 // populations of every lane
-constexpr size_t SMEM_BYTES = size_t(NS) * SN * sizeof(float) + size_t(27) * THREADS * sizeof(float);
+constexpr size_t SMEM_BYTES =
+    size_t(NS) * SN * sizeof(float) + size_t(27) * THREADS * sizeof(float) + size_t(THREADS / 32) * 28 * sizeof(float);
 static_assert(2 * (SMEM_BYTES + 2048) <= 233472, "two CTAs must fit in the 228 KB of an SM");
 
 // Slot of class (k1, k2, k3) in a staged node: the contractions along z and y
@@ -319,6 +325,116 @@ __device__ __forceinline__ void contract_tile(const float* centre, int sx, int s
   }
 }
 
+// The same iterate for one node by the whole warp: lane 5 (oy + 2) + ox + 2
+// contracts the stencil column at (ox, oy) through all three axes, and the
+// lanes' sums are reduced so that lane t < 27 returns population t.  All
+// arguments are the node's (warp-uniform).  Used when few lanes of a warp
+// still iterate: the warp's contraction of all its lanes costs the same
+// however few they are (about 11,000 instructions at N = 4, 1,200 here per node).
+template <int N>
+__device__ __forceinline__ float contract_node_by_warp(const float* centre, int sx, int sxy, const int lo[3],
+                                                       const int hi[3], const int ro[3][3], const float wt[3][3][N],
+                                                       const float bq[3], float ainv, int lane) {
+  const int ox = lane < 25 ? lane % 5 - 2 : 0, oy = lane < 25 ? lane / 5 - 2 : 0;
+  const bool part = lane < 25 && ox >= lo[0] && ox <= hi[0] && oy >= lo[1] && oy <= hi[1];
+  float2 Zp[3][3], Zq[3];
+  float Zs[3], G[3][3];
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+#pragma unroll
+    for (int k2 = 0; k2 < 3; k2++) Zp[i][k2] = make_float2(0.f, 0.f);
+    Zq[i] = make_float2(0.f, 0.f);
+    Zs[i] = 0.f;
+  }
+  basis_rows(bq[2], ainv, G);
+#pragma unroll
+  for (int oz = -H; oz <= H; oz++) {
+    if (oz < lo[2] || oz > hi[2]) continue;
+    float w[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) w[c] = wpick<N>(wt[2][c], ro[2][c], oz);
+    column_node<true, true>(centre + (oz * sxy + oy * sx + ox) * NS, G, w, Zp, Zq, Zs);
+  }
+  float Y[3][9];  // [k1][3 i2 + i3]
+  basis_rows(bq[1], ainv, G);
+#pragma unroll
+  for (int i2 = 0; i2 < 3; i2++) {
+    const float w = wpick<N>(wt[1][i2], ro[1][i2], oy);
+    const float g0 = w * G[i2][0], g1 = w * G[i2][1], g2 = w * G[i2][2];
+#pragma unroll
+    for (int i3 = 0; i3 < 3; i3++) {
+      Y[0][3 * i2 + i3] = fmaf(g2, Zq[i3].y, fmaf(g1, Zq[i3].x, g0 * Zs[i3]));
+      Y[1][3 * i2 + i3] = fmaf(g2, Zp[i3][2].x, fmaf(g1, Zp[i3][1].x, g0 * Zp[i3][0].x));
+      Y[2][3 * i2 + i3] = fmaf(g2, Zp[i3][2].y, fmaf(g1, Zp[i3][1].y, g0 * Zp[i3][0].y));
+    }
+  }
+  float v[32];
+  basis_rows(bq[0], ainv, G);
+#pragma unroll
+  for (int i1 = 0; i1 < 3; i1++) {
+    const float w = wpick<N>(wt[0][i1], ro[0][i1], ox);
+#pragma unroll
+    for (int i23 = 0; i23 < 9; i23++) {
+      const float t = w * fmaf(G[i1][2], Y[2][i23], fmaf(G[i1][1], Y[1][i23], G[i1][0] * Y[0][i23]));
+      v[9 * i1 + i23] = part ? t : 0.f;
+    }
+  }
+#pragma unroll
+  for (int t = 27; t < 32; t++) v[t] = 0.f;
+  // halve the values and the lanes they are summed over: lane t ends with the sum of v[t]
+#pragma unroll
+  for (int h = 16; h > 0; h >>= 1)
+#pragma unroll
+    for (int t = 0; t < h; t++) {
+      const bool up = lane & h;
+      const float give = up ? v[t] : v[t + h], keep = up ? v[t + h] : v[t];
+      v[t] = keep + __shfl_xor_sync(0xffffffffu, give, h);
+    }
+  return v[0];
+}
+
+// The lanes of `live`, one after another, through contract_node_by_warp; each
+// gets its node's populations in acc.  `centre`: the lane's staged node;
+// `scratch`: 27 floats of the warp.
+template <int N>
+__device__ __forceinline__ void contract_live_lanes(unsigned live, const float* staged, int centre, int sx, int sxy,
+                                                    const int lo[3], const int hi[3], const int ro[3][3],
+                                                    const float wt[3][3][N], const float bq[3], float ainv,
+                                                    float* scratch, float acc[27]) {
+  const int lane = (threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z)) & 31;
+#pragma unroll 1
+  for (; live; live &= live - 1) {
+    const int src = __ffs(live) - 1;
+    int lo_s[3], hi_s[3], ro_s[3][3];
+    float wt_s[3][3][N], bq_s[3];
+#pragma unroll
+    for (int ax = 0; ax < 3; ax++) {
+      lo_s[ax] = __shfl_sync(0xffffffffu, lo[ax], src);
+      hi_s[ax] = __shfl_sync(0xffffffffu, hi[ax], src);
+      bq_s[ax] = __shfl_sync(0xffffffffu, bq[ax], src);
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        ro_s[ax][c] = __shfl_sync(0xffffffffu, ro[ax][c], src);
+#pragma unroll
+        for (int k = 0; k < N; k++) wt_s[ax][c][k] = __shfl_sync(0xffffffffu, wt[ax][c][k], src);
+      }
+    }
+    const float a_s = __shfl_sync(0xffffffffu, ainv, src);
+    const float* c_s = staged + __shfl_sync(0xffffffffu, centre, src) * NS;
+    const float r = contract_node_by_warp<N>(c_s, sx, sxy, lo_s, hi_s, ro_s, wt_s, bq_s, a_s, lane);
+    if (lane < 27) scratch[lane] = r;
+    __syncwarp();
+    if (lane == src)
+#pragma unroll
+      for (int t = 0; t < 27; t++) acc[t] = scratch[t];
+    __syncwarp();
+  }
+}
+
+// Live lanes at which the warp serves nodes one by one: the serial iteration
+// costs about 11,000 / 6,500 / 3,000 instructions (N = 4 / 3 / 2), a node by the warp 1,200.
+template <int N> __host__ __device__ constexpr int few_lanes() { return N == 4 ? 5 : N == 3 ? 3 : 1; }
+
 // Partial record of the step sums, updated instead of the context's sums
 // when the kernel runs without a context (kPartials = true; a.sums then
 // points at an array of PARTIALS zeroed records, CTA b adding to record
@@ -542,14 +658,21 @@ __global__ void __launch_bounds__(THREADS, 2) pull_d3q27_tile_kernel(StepArgs<fl
         wl[ax] = __reduce_min_sync(0xffffffffu, done ? H : lo[ax]);
         wh[ax] = __reduce_max_sync(0xffffffffu, done ? -H : hi[ax]);
       }
-      const bool staggered =
-          __all_sync(0xffffffffu, done || (ro[2][1] == wl[2] && ro[2][2] == wl[2] + 1 && ro[2][0] >= wl[2] &&
-                                           ro[2][0] <= wl[2] + 1)) && wh[2] == wl[2] + N;
-      if (!done) {  // floating-point operations of the contractions below
-        const unsigned long long ex = wh[0] - wl[0] + 1, ey = wh[1] - wl[1] + 1, ez = wh[2] - wl[2] + 1;
-        work += ex * ey * (ez * 171 - (staggered ? 114 : 0)) + ex * ey * 171 + ex * 171;
+      const unsigned live = __ballot_sync(0xffffffffu, !done);
+      if (__popc(live) <= few_lanes<N>()) {
+        if (!done) work += 25ull * (5 * 171 + 342);
+        contract_live_lanes<N>(live, sm, sbase, SX, SX * SY, lo, hi, ro, wt, bq, ainv,
+                               sm + NS * SN + 27 * THREADS + (tid >> 5) * 28, acc);
+      } else {
+        const bool staggered =
+            __all_sync(0xffffffffu, done || (ro[2][1] == wl[2] && ro[2][2] == wl[2] + 1 && ro[2][0] >= wl[2] &&
+                                             ro[2][0] <= wl[2] + 1)) && wh[2] == wl[2] + N;
+        if (!done) {  // floating-point operations of the contractions below
+          const unsigned long long ex = wh[0] - wl[0] + 1, ey = wh[1] - wl[1] + 1, ez = wh[2] - wl[2] + 1;
+          work += ex * ey * (ez * 171 - (staggered ? 114 : 0)) + ex * ey * 171 + ex * 171;
+        }
+        contract_tile<N>(sm + sbase * NS, SX, SX * SY, wl, wh, staggered, ro, wt, bq, ainv, acc);
       }
-      contract_tile<N>(sm + sbase * NS, SX, SX * SY, wl, wh, staggered, ro, wt, bq, ainv, acc);
     } else if (!done) {
       // departure points beyond the staged halo: this lane reads global memory
       // and transfers each stencil node into the reference gauge itself

@@ -40,12 +40,14 @@ namespace pond {
 namespace d27e {
 
 using d27::basis_rows;
+using d27::contract_live_lanes;
 using d27::contract_tile;
 using d27::contract_x;
 using d27::contract_y;
 using d27::contract_z;
 using d27::cp_async4;
 using d27::cp_async_wait_all;
+using d27::few_lanes;
 using d27::c_ref27;
 using d27::node_to_ref;
 using d27::rev3;
@@ -63,8 +65,8 @@ constexpr int THREADS = 2 * NODES;
 constexpr int OFF_H = NS * SN;
 constexpr int OFF_OWN = 2 * NS * SN;
 constexpr int OFF_X = OFF_OWN + 27 * THREADS;
-constexpr size_t SMEM_BYTES =
-    size_t(OFF_X) * sizeof(float) + size_t(2 * 5 * NODES) * sizeof(double) + size_t(2 * 2 * NODES) * sizeof(int);
+constexpr int OFF_S = OFF_X + 2 * (2 * 5 * NODES) + 2 * 2 * NODES;  // 28 floats of scratch per warp
+constexpr size_t SMEM_BYTES = size_t(OFF_S + (THREADS / 32) * 28) * sizeof(float);
 static_assert(OFF_X % 2 == 0, "the float64 exchange slots must be 8-byte aligned");
 static_assert(SMEM_BYTES + 3 * 1024 <= 232448, "the tile must fit one CTA per SM");
 
@@ -245,14 +247,21 @@ __global__ void __launch_bounds__(THREADS, 1) pull_d3q27_energy_tile_kernel(Step
         wl[ax] = __reduce_min_sync(0xffffffffu, done ? H : lo[ax]);
         wh[ax] = __reduce_max_sync(0xffffffffu, done ? -H : hi[ax]);
       }
-      const bool staggered =
-          __all_sync(0xffffffffu, done || (ro[2][1] == wl[2] && ro[2][2] == wl[2] + 1 && ro[2][0] >= wl[2] &&
-                                           ro[2][0] <= wl[2] + 1)) && wh[2] == wl[2] + N;
-      if (!done) {
-        const unsigned long long ex = wh[0] - wl[0] + 1, ey = wh[1] - wl[1] + 1, ez = wh[2] - wl[2] + 1;
-        work += ex * ey * (ez * 171 - (staggered ? 114 : 0)) + ex * ey * 171 + ex * 171;
+      const unsigned live = __ballot_sync(0xffffffffu, !done);
+      if (__popc(live) <= few_lanes<N>()) {
+        if (!done) work += 25ull * (5 * 171 + 342);
+        contract_live_lanes<N>(live, sd, sbase, SX, SX * SY, lo, hi, ro, wt, bq, ainv,
+                               sm + OFF_S + (tid >> 5) * 28, acc);
+      } else {
+        const bool staggered =
+            __all_sync(0xffffffffu, done || (ro[2][1] == wl[2] && ro[2][2] == wl[2] + 1 && ro[2][0] >= wl[2] &&
+                                             ro[2][0] <= wl[2] + 1)) && wh[2] == wl[2] + N;
+        if (!done) {
+          const unsigned long long ex = wh[0] - wl[0] + 1, ey = wh[1] - wl[1] + 1, ez = wh[2] - wl[2] + 1;
+          work += ex * ey * (ez * 171 - (staggered ? 114 : 0)) + ex * ey * 171 + ex * 171;
+        }
+        contract_tile<N>(sd + sbase * NS, SX, SX * SY, wl, wh, staggered, ro, wt, bq, ainv, acc);
       }
-      contract_tile<N>(sd + sbase * NS, SX, SX * SY, wl, wh, staggered, ro, wt, bq, ainv, acc);
     } else if (!done) {
       // departure points beyond the staged halo: global memory, each stencil
       // node transferred into the reference gauge by this lane
