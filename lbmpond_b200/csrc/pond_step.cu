@@ -195,6 +195,13 @@ template <int LAT, int N, typename R> static void launch_point(const StepArgs<R>
   }
 }
 
+// CTAs of the GAP2 step: the windows of 128 nodes, at most the six per SM that
+// are resident (4M nodes, float32: 0.26 ms per step; a CTA per window 0.34 ms,
+// most of it the CTAs' additions to the step's sums).  NONUNIFORM3 keeps a CTA
+// per window: its node setup leaves fewer warps to hide the loop's barriers
+// (4M nodes: 0.51 ms, 0.73 ms looped).
+static int gap2_ctas(int nx) { return (nx + 127) / 128 < 148 * 6 ? (nx + 127) / 128 : 148 * 6; }
+
 // D1Q5, one step of a 1D grid of at most W1D_MAX nodes with a warp per node:
 // there the step is one node's chain of iterations, however many nodes; above
 // it the one-thread-per-node kernels do more nodes per instruction.  Measured,
@@ -362,7 +369,7 @@ template <typename R> static int launch_typed(pond_ctx* c, const void* const* in
           pull_1d_scheme_kernel<POND_WENO5, R><<<(a.nx + 127) / 128, 128, 0, s>>>(a);
           break;
         case POND_GAP2:
-          pull_1d_mesh_kernel<POND_GAP2, R><<<(a.nx + 127) / 128, 128, 0, s>>>(a);
+          pull_1d_mesh_kernel<POND_GAP2, R><<<gap2_ctas(a.nx), 128, 0, s>>>(a);
           break;
         case POND_NONUNIFORM3:
           pull_1d_mesh_kernel<POND_NONUNIFORM3, R><<<(a.nx + 127) / 128, 128, 0, s>>>(a);

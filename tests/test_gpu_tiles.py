@@ -144,6 +144,36 @@ def test_d1q5_warp_and_thread_per_node(orc, pond, nx, kind, bc, interp, precisio
         assert abs(d["mass"] - ref.rho.sum()) <= 1e-9 * ref.rho.sum()
 
 
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_gap2_windows_and_long_departures(orc, pond, precision):
+    """More windows than CTAs, and nodes whose departure points pass their nearest active neighbours."""
+    nx = 120001
+    rho, g = smooth_state((nx, 1, 1), 1, seed=4, modes=1, T0=0.02, du=0.02, dT=0.002)
+    rng = np.random.default_rng(4)
+    mask = (rng.random(nx) < 0.6).astype(np.uint8)
+    mask[1000:1400] = 0
+    mask[0] = 1
+    g[0, 40000:60000] += 1.3  # |v| up to 1.8 nodes
+    f = perturbed_populations(orc, 0, rho, g, seed=4, eps=0.01)
+    if precision == "fp32":
+        rho, g, f = (a.astype(np.float32).astype(float) for a in (rho, g, f))
+    with pond.Solver(lattice=0, shape=(nx, 1, 1), interp=9, precision=precision, tau=0.8, max_iter=3) as s:
+        s.set_mask(mask)
+        s.set_state(rho, g, f=f)
+        s.step(1)
+        out = s.get_state()
+    ref, niter, nc = orc.step_mesh(orc.State(f, rho, g), nx, interp=orc.GAP2, mask=mask, tau=0.8, max_iter=3)
+    if precision == "fp32":
+        # across the two jumps of u the quartic basis is taken 9 speeds out: terms of size 500 f cancel, which
+        # float32 cannot hold to its tolerance; the stencils there reach a few active nodes
+        keep = np.ones(nx, bool)
+        for jump in (40000, 60000):
+            keep[jump - 64:jump + 64] = False
+        out = tuple(a[..., keep] for a in out)
+        ref = orc.State(ref.f[:, keep], ref.rho[keep], ref.g[:, keep])
+    _compare(out, ref, TOL[precision], "gap2")
+
+
 def test_noalloc_records_shared_by_ctas(pond):
     """A grid of more CTAs than partial-sum records: the step's sums against the context's."""
     import torch
