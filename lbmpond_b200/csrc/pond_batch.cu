@@ -2,7 +2,8 @@
 // advanced by persistent kernel launches replayed from a CUDA graph.
 //
 // Layout.  At creation the problems are packed (best fit, longest first)
-// into bins of at most BIN_CAP = 6144 nodes and BIN_SEGS problems; the
+// into bins of at most BIN_CAP = 6144 nodes and BIN_SEGS problems, smaller
+// where those would leave SMs without one (choose_bins); the
 // device state is stored bin after bin, SoA: f[5][S], rho, u, T (float32),
 // every bin starting on a 4-node (16-byte) boundary, S the padded total.
 // Host set/get calls translate to and from the caller's problem order.
@@ -201,6 +202,91 @@ __device__ __forceinline__ float pull_population(int k, const float* sf, const f
   return g;
 }
 
+// Window nodes of a population, and how far the windows of a node's
+// populations may lie apart for pull_near.
+template <int SCHEME> __host__ __device__ constexpr int window_nodes() { return SCHEME == POND_WENO5 ? 5 : 4; }
+constexpr int NEAR = 2;
+// Problems with more than 1 / HOT_SHARE of their nodes above c = HOT_C, where
+// the fastest populations' windows lie too far apart (2.86 c rounds to two
+// nodes at 0.525), go the general way as a whole: lanes of both kinds in one
+// warp cost the sum of both (the log-uniform set ran 6 % slower with the
+// choice left to each node).
+constexpr float HOT_C = 0.5f;
+constexpr int HOT_SHARE = 8;
+constexpr int HOT_EVERY = 8;  // steps of a launch between counts
+
+// New values of all five populations, one lane, when their windows start
+// within NEAR nodes of each other: every node of the union (window + NEAR
+// nodes) is read once and transferred for all populations at once -- the
+// powers of the five normalised speeds are shared, and the +- pairs of
+// populations share their common factor and run as two-wide operations --
+// about 650 instructions instead of 25 separate transfers of 55.  Every product
+// is rounded as in transfer_row, so both ways give the same bits (tubes with
+// nodes at the iteration cap amplify a last-digit difference to percents
+// within 400 steps).  Returns false, with nothing written, when the windows lie
+// further apart or a node's gauge is so far off that a basis value could overflow.
+template <int SCHEME>
+__device__ __forceinline__ bool pull_near(const float* sf, const float* su, const float* sc, int ps, int n, int xl,
+                                          const double vk[5], float Uf, float invC, float fn[5]) {
+  constexpr int W = window_nodes<SCHEME>(), M = W + NEAR;
+  constexpr double e1s = EC1 * EC1, e2s = EC2 * EC2;
+  float off[5];
+  int d[5];
+#pragma unroll
+  for (int k = 0; k < 5; k++) d[k] = window<SCHEME>(double(xl) - vk[k], off[k]);
+  const int first = min(min(min(d[0], d[1]), min(d[2], d[3])), d[4]);
+  const int last = max(max(max(d[0], d[1]), max(d[2], d[3])), d[4]);
+  if ((long long)last - first > NEAR) return false;
+  float T0[M];
+  float2 Ta[M], Tb[M];  // populations 1, 2 and 3, 4
+  bool ok = true;
+#pragma unroll
+  for (int m = 0; m < M; m++) {
+    const int q = ps + min(max(first + m, 0), n - 1);
+    const float s = __fmul_rn(__fsub_rn(su[q], Uf), invC), r = __fmul_rn(sc[q], invC);
+    ok = ok && fabsf(s) < 1e8f && fabsf(r) < 1e8f;
+    T0[m] = 0.f;
+    Ta[m] = Tb[m] = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int b = 0; b < 5; b++) {
+      const float f = sf[b * BIN_CAP + q];
+      const float y = fmaf(r, float(Lattice<POND_D1Q5>::xi1(b)), s), y2 = __fmul_rn(y, y);
+      const float p1 = __fsub_rn(y2, float(e1s)), p2 = __fsub_rn(y2, float(e2s));
+      const float g0 = __fmul_rn(float(1.0 / (e1s * e2s)), p1);
+      const float ga = __fmul_rn(float(1.0 / (2.0 * e1s * (e1s - e2s))), p2);
+      const float gb = __fmul_rn(float(1.0 / (2.0 * e2s * (e2s - e1s))), p1);
+      const float2 ff = make_float2(f, f), yy = make_float2(y, y), yy2 = make_float2(y2, y2);
+      T0[m] = fmaf(__fmul_rn(g0, __fsub_rn(y2, float(e2s))), f, T0[m]);
+      const float2 qa = __ffma2_rn(make_float2(float(EC1), -float(EC1)), yy, yy2);
+      const float2 qb = __ffma2_rn(make_float2(float(EC2), -float(EC2)), yy, yy2);
+      Ta[m] = __ffma2_rn(__fmul2_rn(make_float2(ga, ga), qa), ff, Ta[m]);
+      Tb[m] = __ffma2_rn(__fmul2_rn(make_float2(gb, gb), qb), ff, Tb[m]);
+    }
+  }
+  if (!ok) return false;
+#pragma unroll
+  for (int k = 0; k < 5; k++) {
+    const int sh = d[k] - first;  // 0 .. NEAR
+    float w[W];
+#pragma unroll
+    for (int j = 0; j < W; j++) {
+      const auto at = [&](int m) { return k == 0 ? T0[m] : k == 1 ? Ta[m].x : k == 2 ? Ta[m].y : k == 3 ? Tb[m].x : Tb[m].y; };
+      w[j] = sh == 0 ? at(j) : sh == 1 ? at(j + 1) : at(j + 2);
+    }
+    if constexpr (SCHEME == POND_WENO5) {
+      fn[k] = weno5(w, off[k]);
+    } else {
+      float l[4];
+      lagr4(off[k], l);
+      float g = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; j++) g = fmaf(l[j], w[j], g);
+      fn[k] = g;
+    }
+  }
+  return true;
+}
+
 // cnew.calcMoments (float64), the T < 0 guard and isConv; then c0 = cnew.
 // Returns true when the iteration has converged.
 __device__ __forceinline__ bool moments_and_test(const Args& a, const float fn[5], const double vk[5], Node& s) {
@@ -229,8 +315,8 @@ __device__ __forceinline__ bool moments_and_test(const Args& a, const float fn[5
   return ok;
 }
 
-// The problem holding bin node x: s_seg[j] <= x < s_seg[j + 1].
-__device__ __forceinline__ void locate(const int* s_seg, int nseg, int x, int& ps, int& n) {
+// The problem holding bin node x: s_seg[j] <= x < s_seg[j + 1]; returns j.
+__device__ __forceinline__ int locate(const int* s_seg, int nseg, int x, int& ps, int& n) {
   int lo = 0, hi = nseg;
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
@@ -238,6 +324,7 @@ __device__ __forceinline__ void locate(const int* s_seg, int nseg, int x, int& p
   }
   ps = s_seg[lo];
   n = s_seg[lo + 1] - ps;
+  return lo;
 }
 
 // rho of staged node q: the sum of its populations (the stored rho is that
@@ -342,6 +429,7 @@ __global__ void __launch_bounds__(NT, 1) batch_kernel(Args a) {
   float* sT = sm + 6 * BIN_CAP;  // T
   float* sc = sm + 7 * BIN_CAP;  // c = sqrts(T / TLat)
   __shared__ int s_seg[BIN_SEGS + 1];
+  __shared__ int s_hot[BIN_SEGS];  // nodes of each problem with c > HOT_C
   __shared__ Node s_hard[HARD_MAX];
   __shared__ int s_bin, s_next, s_nhard, s_hnext;
   __shared__ __align__(8) unsigned long long s_bar;
@@ -373,6 +461,8 @@ __global__ void __launch_bounds__(NT, 1) batch_kernel(Args a) {
         bulk_g2s(su, a.u + off, bytes, &s_bar);
         bulk_g2s(sT, a.T + off, bytes, &s_bar);
       }
+      const bool count_hot = step % HOT_EVERY == 0;
+      if (count_hot && tid < BIN_SEGS) s_hot[tid] = 0;
       const bool staged = mbar_wait(&s_bar, phase & 1u);
       phase++;
       if (__syncthreads_or(!staged)) {  // a copy did not land: report, give it one more bounded wait, leave
@@ -382,11 +472,26 @@ __global__ void __launch_bounds__(NT, 1) batch_kernel(Args a) {
         }
         return;
       }
-      for (int i = tid; i < fill; i += NT) {
+      for (int i0 = tid - lane; i0 < fill; i0 += NT) {  // warp-uniform
+        const int i = i0 + lane;
+        bool hot = false;
+        if (i < fill) {
 #pragma unroll
-        for (int k = 0; k < 5; k++) sf[k * BIN_CAP + i] = finite_or_zero(sf[k * BIN_CAP + i]);
-        const float T = sT[i];
-        sc[i] = copysignf(sqrtf(fabsf(T) * float(1.0 / L::TLat)), T);
+          for (int k = 0; k < 5; k++) sf[k * BIN_CAP + i] = finite_or_zero(sf[k * BIN_CAP + i]);
+          const float T = sT[i], c = copysignf(sqrtf(fabsf(T) * float(1.0 / L::TLat)), T);
+          sc[i] = c;
+          hot = c > HOT_C;
+        }
+        const unsigned hots = count_hot ? __ballot_sync(0xffffffffu, hot) : 0;
+        if (hots) {
+          int p0, n0;
+          const int j = locate(s_seg, nseg, i0, p0, n0);
+          if (i0 + 32 <= p0 + n0) {  // one problem
+            if (lane == 0) atomicAdd(&s_hot[j], __popc(hots));
+          } else if (hot) {
+            atomicAdd(&s_hot[locate(s_seg, nseg, i, p0, n0)], 1);
+          }
+        }
       }
       if (tid == 0) { s_next = NT; s_nhard = 0; s_hnext = 0; }
       __syncthreads();
@@ -394,9 +499,11 @@ __global__ void __launch_bounds__(NT, 1) batch_kernel(Args a) {
       // phase 1: one lane per node
       Node s;
       int ps = 0, n = 1;
+      bool cold = false;  // the problem's windows mostly lie near each other
       if (tid < fill) {
         load_node(sf, su, sT, tid, s);
-        locate(s_seg, nseg, tid, ps, n);
+        const int j = locate(s_seg, nseg, tid, ps, n);
+        cold = HOT_SHARE * s_hot[j] <= n;
       } else {
         s.x = fill;
       }
@@ -408,8 +515,9 @@ __global__ void __launch_bounds__(NT, 1) batch_kernel(Args a) {
         float fn[5];
 #pragma unroll
         for (int k = 0; k < 5; k++) vk[k] = C * L::xi1(k) + s.U;
+        if (!cold || !pull_near<SCHEME>(sf, su, sc, ps, n, s.x - ps, vk, Uf, invC, fn))
 #pragma unroll
-        for (int k = 0; k < 5; k++) fn[k] = pull_population<SCHEME>(k, sf, su, sc, ps, n, s.x - ps, vk[k], Uf, invC);
+          for (int k = 0; k < 5; k++) fn[k] = pull_population<SCHEME>(k, sf, su, sc, ps, n, s.x - ps, vk[k], Uf, invC);
         const bool ok = moments_and_test(a, fn, vk, s);
         if (!ok && s.niter < a.max_iter) {
           if (s.niter != a.lane_cap) continue;
@@ -425,7 +533,8 @@ __global__ void __launch_bounds__(NT, 1) batch_kernel(Args a) {
         const int x = atomicAdd(&s_next, 1);
         if (x < fill) {
           load_node(sf, su, sT, x, s);
-          locate(s_seg, nseg, x, ps, n);
+          const int j = locate(s_seg, nseg, x, ps, n);
+          cold = HOT_SHARE * s_hot[j] <= n;
         } else {
           s.x = fill;
         }
@@ -511,8 +620,9 @@ struct pond_batch {
   int interp = POND_WENO5;
   double tau = 0.9, tol_abs = 1e-7, tol_rel = 1e-6;
   int max_iter = 100;
-  int threads = 768;   // threads per CTA (autotuned)
-  int lane_cap = 4;    // phase-1 iterations per node (autotuned)
+  int threads = 512;   // threads per CTA (default_tile, or the caller's)
+  int lane_cap = 8;    // phase-1 iterations per node
+  bool tile_given = false;  // by pond_batch_set_tile or the autotuner
   int grid = 0;
   cudaStream_t stream = nullptr;
   float* f = nullptr;
@@ -615,12 +725,10 @@ static int chunk_graph(pond_batch* b, int k) {
   return POND_OK;
 }
 
-// Best-fit packing of the problems, longest first, into bins of at most
-// BIN_CAP nodes and BIN_SEGS problems.
-static void pack(const int32_t* lengths, int P, std::vector<std::vector<int>>& bins) {
-  std::vector<int> order(P);
-  std::iota(order.begin(), order.end(), 0);
-  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return lengths[x] > lengths[y]; });
+// Best-fit packing of the problems, in `order` (longest first), into bins of
+// at most `cap` nodes and BIN_SEGS problems; returns the nodes of the fullest.
+static int pack(const int32_t* lengths, const std::vector<int>& order, int cap, std::vector<std::vector<int>>& bins) {
+  bins.clear();
   std::set<std::pair<int, int>> room;  // (free nodes, bin) of bins with a free problem slot
   std::vector<int> free_nodes;
   for (int p : order) {
@@ -630,7 +738,7 @@ static void pack(const int32_t* lengths, int P, std::vector<std::vector<int>>& b
     if (it == room.end()) {
       bi = (int)bins.size();
       bins.emplace_back();
-      free_nodes.push_back(BIN_CAP);
+      free_nodes.push_back(cap);
     } else {
       bi = it->second;
       room.erase(it);
@@ -638,6 +746,34 @@ static void pack(const int32_t* lengths, int P, std::vector<std::vector<int>>& b
     bins[bi].push_back(p);
     free_nodes[bi] -= l;
     if ((int)bins[bi].size() < BIN_SEGS && free_nodes[bi] > 0) room.insert({free_nodes[bi], bi});
+  }
+  return cap - *std::min_element(free_nodes.begin(), free_nodes.end());
+}
+
+// The bins of a batch.  Where bins of BIN_CAP nodes do not even fill the SMs
+// once, smaller ones (no smaller than the longest problem) put a bin on every
+// SM: 43k nodes in 47 bins instead of 7 run 0.035 instead of 0.126 ms per step,
+// 571k nodes in 145 instead of 94 0.070 instead of 0.108.  With more bins than
+// SMs BIN_CAP stays: evening out the last round (2.2M nodes, 444 bins instead
+// of 361) gains 7 % where the work of a bin-step dominates, but a bin-step also
+// costs its hardest node's chain, and on the log-uniform Riemann set, where
+// that dominates, more bins cost 12-16 %.
+static void choose_bins(const int32_t* lengths, int P, long long nodes, int sms, std::vector<std::vector<int>>& bins) {
+  std::vector<int> order(P);
+  std::iota(order.begin(), order.end(), 0);
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return lengths[x] > lengths[y]; });
+  pack(lengths, order, BIN_CAP, bins);
+  if ((int)bins.size() >= sms) return;
+  const int even = std::max(lengths[order[0]], (int)((nodes + sms - 1) / sms));
+  for (const double slack : {1.0, 1.005, 1.01, 1.02, 1.04, 1.08, 1.15, 1.3}) {
+    const int cap = (int)(even * slack);
+    if (cap >= BIN_CAP) return;
+    std::vector<std::vector<int>> tried;
+    pack(lengths, order, cap, tried);
+    if ((int)tried.size() <= sms) {
+      bins.swap(tried);
+      return;
+    }
   }
 }
 
@@ -680,8 +816,10 @@ int pond_batch_create(int nproblems, const int32_t* lengths, int interp, double 
   }
   cudaError_t e = cudaSetDevice(device);
   if (e != cudaSuccess) return cuda_fail(e, "cudaSetDevice");
+  int nsm = 148;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
   std::vector<std::vector<int>> bins;
-  batch::pack(lengths, nproblems, bins);
+  batch::choose_bins(lengths, nproblems, Ltot, nsm, bins);
   pond_batch* b = new pond_batch();
   b->device = device; b->P = nproblems; b->B = (int)bins.size(); b->Ltot = Ltot; b->interp = interp;
   b->tau = tau; b->tol_abs = tol_abs; b->tol_rel = tol_rel; b->max_iter = max_iter;
@@ -703,8 +841,6 @@ int pond_batch_create(int nproblems, const int32_t* lengths, int interp, double 
   seg_first[b->B] = (int)segs.size();
   const long long S = bin_off[b->B];
   b->stride = S;
-  int nsm = 148;
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
   b->grid = std::min(b->B, nsm);  // one resident CTA per SM (a bin fills most of shared memory)
   bool ok = cudaMalloc(&b->f, 5 * S * sizeof(float)) == cudaSuccess &&
             cudaMalloc(&b->rho, S * sizeof(float)) == cudaSuccess &&
@@ -753,11 +889,22 @@ int pond_batch_create(int nproblems, const int32_t* lengths, int interp, double 
 int64_t pond_batch_nodes(const pond_batch* b) { return b ? b->Ltot : 0; }
 int32_t pond_batch_bins(const pond_batch* b) { return b ? b->B : 0; }
 
+// The tile of a state nobody tuned for.  Where the windows lie near each other
+// 512 threads keep pull_near's values in registers (4096 tubes with density
+// ratios up to 4, WENO5 / cubic: 0.73 / 0.51 ms per step against 0.80 / 0.55
+// with 768); where they do not, more threads hide the general way better
+// (log-uniform tubes: 4.37 / 4.32 with 512, 4.09 / 3.92 with 768).
+static void default_tile(pond_batch* b, long long hot) {
+  if (b->tile_given) return;
+  b->threads = 4 * hot > b->Ltot ? 768 : 512;
+  b->lane_cap = 8;
+}
+
 int pond_batch_set_state(pond_batch* b, const double* rho, const double* u, const double* T) {
   if (!b || !rho || !u || !T) return set_error(POND_ERR_ARG, "pond_batch_set_state: null argument");
   const long long n = b->stride;
   std::vector<float> fb(5 * n), rb(n), ub(n), tb(n);
-  long long src = 0;
+  long long src = 0, hot = 0;
   for (int p = 0; p < b->P; p++) {
     const long long dst = b->pos[p];
     for (int i = 0; i < b->len[p]; i++, src++) {
@@ -765,6 +912,7 @@ int pond_batch_set_state(pond_batch* b, const double* rho, const double* u, cons
       if (!(std::isfinite(r) && std::isfinite(v) && t > 0 && std::isfinite(t)))
         return set_error(POND_ERR_ARG, "problem %d node %d: rho and u must be finite and T > 0", p, i);
       rb[dst + i] = (float)r; ub[dst + i] = (float)v; tb[dst + i] = (float)t;
+      hot += t > batch::HOT_C * batch::HOT_C;
       for (int k = 0; k < 5; k++) fb[k * n + dst + i] = (float)(lattice_weight_t<POND_D1Q5>(k) * r);
     }
   }
@@ -776,6 +924,7 @@ int pond_batch_set_state(pond_batch* b, const double* rho, const double* u, cons
   if (e == cudaSuccess) e = cudaMemcpy(b->T, tb.data(), n * sizeof(float), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemset(b->istep_dev, 0, sizeof(int));
   b->istep = 0;
+  default_tile(b, hot);
   return e == cudaSuccess ? POND_OK : cuda_fail(e, "pond_batch_set_state");
 }
 
@@ -882,6 +1031,7 @@ int pond_batch_set_tile(pond_batch* b, int threads, int lane_cap) {
     return set_error(POND_ERR_ARG, "tile: threads per CTA 256, 512, 768 or 1024 and lane_cap >= 1");
   b->threads = threads;
   b->lane_cap = lane_cap;
+  b->tile_given = true;
   return POND_OK;
 }
 
@@ -948,6 +1098,7 @@ int pond_batch_autotune(pond_batch* b, int probe_steps, const int32_t* tiles, in
   const bool ok = st == POND_OK && best_c >= 0;
   b->threads = ok ? tiles[2 * best_c] : saved[0];
   b->lane_cap = ok ? tiles[2 * best_c + 1] : saved[1];
+  b->tile_given = b->tile_given || ok;
   batch::drop_graph(b);
   if (best) *best = best_c;
   return st;
