@@ -73,3 +73,22 @@ def test_tiles_and_packings_agree_bit_for_bit(pond):
     sl = slice(int(np.sum(LENGTHS[:p])), int(np.sum(LENGTHS[:p + 1])))
     for x, y in zip(full, run(LENGTHS[p:p + 1], sl)):
         assert np.array_equal(x[..., sl], y)
+
+
+@pytest.mark.parametrize("count", [3, 90])
+def test_read_back_puts_every_node_in_its_place(pond, count):
+    """Both read-backs (plain; chunked over threads above 200,000 nodes) on problems of uneven length."""
+    from lbmpond_b200.batch import Batch
+    rng = np.random.default_rng(count)
+    lengths = rng.integers(1, 4097, count * 2)
+    lengths[:count] = rng.integers(3000, 4097, count)
+    n = int(lengths.sum())
+    assert (n > 200000) == (count == 90)
+    rho, u, T = (rng.uniform(0.5, 1.5, n).astype(np.float32).astype(float) for _ in range(3))
+    with Batch(lengths) as b:
+        b.set_state(rho, u, T)
+        for _ in range(2):
+            f, r, uu, tt = b.get_state()
+            assert np.array_equal(r, rho) and np.array_equal(uu, u) and np.array_equal(tt, T)
+            w = f[:, 0] / rho[0]
+            assert np.abs(f - w[:, None] * rho).max() <= 1e-6
