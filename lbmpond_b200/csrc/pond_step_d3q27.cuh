@@ -9,10 +9,11 @@
 //    node's 27 populations are contiguous and 16-byte aligned (a 28-float
 //    stride, 86 KB), so a lane fetches a stencil node with seven 16-byte
 //    loads, and the 28-word stride puts the eight lanes of every 16-byte load
-//    phase on distinct banks.  Two CTAs share an SM (100 KB and 128 threads
+//    phase on distinct banks.  Two CTAs share an SM (110 KB and 128 threads
 //    of 255 registers each): one stages while the other iterates, and neither
 //    waits for the other's slowest warp.  Each staging thread copies whole
-//    nodes and transfers them itself (no gauge planes in shared memory).
+//    nodes with their gauges, all copies in flight at once, and transfers them
+//    itself.
 //    Boundary resolution (periodic wrap, clamp, mirror with population
 //    reversal), the reference's dropping of non-finite terms and the square
 //    root of T are applied while staging;
@@ -43,16 +44,18 @@
 //    (slot27): 45 instructions per stencil node instead of 81, for the same
 //    81 multiply-adds with the same roundings.
 //
-// What bounds it: the 128 B/clk of shared memory.  A stencil node costs 28
-// wavefronts per warp and 20-23 cycles of the SM's FMA pipes, so an iteration
-// of 125 nodes takes at least 3,500 cycles per warp of its SM: 20 ms of the
-// 30.0 ms that a 256^3 step of a half-uniform blast takes (46.1 ms in the
-// earlier form: 32 x 4 x 2 tiles, one CTA of 256 threads per SM, scalar
-// multiply-adds, rolled z offsets).  At 128^3, by ncu: shared-memory
-// wavefronts 70 % of peak, FMA pipe 52 % (the earlier form 40 %), issue slots
-// 52 %, 2.49 G warp instructions.
-//  * a lane whose departure points leave the +-2 halo (|u| + sqrt(T/TLat) >= 1
-//    along an axis) runs that iteration from global memory instead.
+// What bounds it: the 128 B/clk of shared memory and, at two warps per
+// scheduler, latency.  A stencil node costs 28 wavefronts per warp and 20-23
+// cycles of the SM's FMA pipes, so an iteration of 125 nodes takes at least
+// 3,500 cycles per warp of its SM: 19 ms of the 27.9 ms that a 256^3 step of a
+// half-uniform blast takes (46.1 ms in the earlier form: 32 x 4 x 2 tiles, one
+// CTA of 256 threads per SM, scalar multiply-adds, rolled z offsets).  Of that
+// the first form of this kernel took 30.0; walking k3 outermost in the column
+// node (1.0 ms), copying the gauges with the populations instead of loading
+// them node by node (0.4), transferring staged nodes on pairs, keeping the
+// tile's own populations while staging and shorter float64 sums (0.3) the rest.
+// At 128^3, by ncu, in the first form: shared-memory wavefronts 70 % of peak,
+// FMA pipe 52 % (the earlier form 40 %), issue slots 52 %.
 #pragma once
 #include "pond_step_point.cuh"
 
@@ -69,7 +72,8 @@ constexpr int THREADS = TX * TY * TZ;
 // lanes of each 16-byte load phase on distinct banks), then the iterate's
 // populations of every lane
 constexpr size_t SMEM_BYTES =
-    size_t(NS) * SN * sizeof(float) + size_t(27) * THREADS * sizeof(float) + size_t(THREADS / 32) * 28 * sizeof(float);
+    size_t(NS) * SN * sizeof(float) + size_t(27) * THREADS * sizeof(float) + size_t(THREADS / 32) * 28 * sizeof(float) +
+    size_t(3) * SN * sizeof(float);
 static_assert(2 * (SMEM_BYTES + 2048) <= 233472, "two CTAs must fit in the 228 KB of an SM");
 
 // Slot of class (k1, k2, k3) in a staged node: the contractions along z and y
@@ -77,7 +81,7 @@ static_assert(2 * (SMEM_BYTES + 2048) <= 233472, "two CTAs must fit in the 228 K
 // classes k1 = +, - of each (k2, k3) are neighbours (slots 0-17), the k1 = 0
 // classes k2 = +, - of each k3 (slots 18-23) and the three of k2 = 0 are last.
 __host__ __device__ constexpr int slot27(int k1, int k2, int k3) {
-  return k1 > 0 ? 2 * (3 * k2 + k3) + (k1 - 1) : k2 > 0 ? 18 + 2 * k3 + (k2 - 1) : 24 + k3;
+  return k1 > 0 ? 2 * (3 * k3 + k2) + (k1 - 1) : k2 > 0 ? 18 + 2 * k3 + (k2 - 1) : 24 + k3;
 }
 __host__ __device__ constexpr int slot27(int t) { return slot27(t / 9, (t / 3) % 3, t % 3); }
 
@@ -135,6 +139,144 @@ template <typename R> __device__ __forceinline__ void node_to_ref(R v[27], const
       }
     }
   }
+}
+
+// node_to_ref of a staged node in its slots, non-finite populations counted
+// as 0 (all of them when !ok): pairs of classes k1 = +, - through the z and y
+// passes and pairs of target classes i1 = +, - in the x pass, 153
+// instructions for the 243 multiply-adds.  `raw` (null, or the node's column
+// of the iterates, `stride` floats apart) gets the populations as they were.
+__device__ __forceinline__ void staged_to_ref(float* node, bool ok, const float s[3], const float r[3], float* raw,
+                                              int stride) {
+  float e[28];
+  float4* s4 = reinterpret_cast<float4*>(node);
+#pragma unroll
+  for (int q = 0; q < 7; q++) {
+    const float4 w = s4[q];
+    e[4 * q] = w.x; e[4 * q + 1] = w.y; e[4 * q + 2] = w.z; e[4 * q + 3] = w.w;
+  }
+  if (raw)
+#pragma unroll
+    for (int t = 0; t < 27; t++) raw[t * stride] = e[slot27(t)];
+#pragma unroll
+  for (int q = 0; q < 27; q++) e[q] = (ok && fabsf(e[q]) <= 3.402823466e38f) ? e[q] : 0.f;
+  float B[3][3];
+  float2 P[3][3], Q[3];  // [k2][i3] of k1 = +, -; [i3] of k1 = 0, k2 = +, -
+  float S[3];            // [i3] of k1 = k2 = 0
+  basis_rows(s[2], r[2], B);
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    const auto row = [&](int slot, int step) {  // sum_k3 B[i][k3] of the pairs at slot, slot + step, ..
+      float2 o = __fmul2_rn(make_float2(B[i][0], B[i][0]), make_float2(e[slot], e[slot + 1]));
+      o = __ffma2_rn(make_float2(B[i][1], B[i][1]), make_float2(e[slot + step], e[slot + step + 1]), o);
+      return __ffma2_rn(make_float2(B[i][2], B[i][2]), make_float2(e[slot + 2 * step], e[slot + 2 * step + 1]), o);
+    };
+#pragma unroll
+    for (int k2 = 0; k2 < 3; k2++) P[k2][i] = row(slot27(1, k2, 0), slot27(1, 0, 1) - slot27(1, 0, 0));
+    Q[i] = row(slot27(0, 1, 0), slot27(0, 1, 1) - slot27(0, 1, 0));
+    S[i] = fmaf(B[i][2], e[26], fmaf(B[i][1], e[25], B[i][0] * e[24]));
+  }
+  basis_rows(s[1], r[1], B);
+  float2 P2[3][3];  // [i2][i3] of k1 = +, -
+  float Z[3][3];    // [i2][i3] of k1 = 0
+#pragma unroll
+  for (int i2 = 0; i2 < 3; i2++)
+#pragma unroll
+    for (int i3 = 0; i3 < 3; i3++) {
+      const float b0 = B[i2][0], b1 = B[i2][1], b2 = B[i2][2];
+      P2[i2][i3] = __ffma2_rn(make_float2(b2, b2), P[2][i3],
+                              __ffma2_rn(make_float2(b1, b1), P[1][i3], __fmul2_rn(make_float2(b0, b0), P[0][i3])));
+      Z[i2][i3] = fmaf(b2, Q[i3].y, fmaf(b1, Q[i3].x, b0 * S[i3]));
+    }
+  basis_rows(s[0], r[0], B);
+  const float2 c0 = make_float2(B[1][0], B[2][0]), c1 = make_float2(B[1][1], B[2][1]), c2 = make_float2(B[1][2], B[2][2]);
+#pragma unroll
+  for (int i2 = 0; i2 < 3; i2++)
+#pragma unroll
+    for (int i3 = 0; i3 < 3; i3++) {
+      const float z = Z[i2][i3], p = P2[i2][i3].x, m = P2[i2][i3].y;
+      e[slot27(0, i2, i3)] = fmaf(B[0][2], m, fmaf(B[0][1], p, B[0][0] * z));
+      const float2 o = __ffma2_rn(c2, make_float2(m, m), __ffma2_rn(c1, make_float2(p, p), __fmul2_rn(c0, make_float2(z, z))));
+      e[slot27(1, i2, i3)] = o.x;
+      e[slot27(2, i2, i3)] = o.y;
+    }
+  e[27] = 0.f;
+#pragma unroll
+  for (int q = 0; q < 7; q++) s4[q] = make_float4(e[4 * q], e[4 * q + 1], e[4 * q + 2], e[4 * q + 3]);
+}
+
+// Queue the copies of global node g's populations into the slots of a staged
+// node (`rv`: axes mirrored there, which reverses the classes along them).
+__device__ __forceinline__ void copy_node(const float* f, long long N, long long g, const bool rv[3], float* node) {
+  if (!(rv[0] || rv[1] || rv[2])) {
+    // in the stored order, one addition per population
+    constexpr int cls[27] = {0, 9, 3, 1, 12, 10, 4, 13, 18, 21, 19, 22, 6, 7, 15, 16, 2, 11, 5, 14, 24, 25, 20, 23, 8, 17, 26};
+    const float* src = f + g;
+#pragma unroll
+    for (int q = 0; q < 27; q++) {
+      cp_async4(node + slot27(cls[q]), src);
+      src += N;
+    }
+    return;
+  }
+#pragma unroll
+  for (int t = 0; t < 27; t++) {
+    int cx = t / 9, cy = (t / 3) % 3, cz = t % 3;
+    if (rv[0]) cx = rev3(cx);
+    if (rv[1]) cy = rev3(cy);
+    if (rv[2]) cz = rev3(cz);
+    cp_async4(node + slot27(t), f + (long long)c_ref27[cx * 9 + cy * 3 + cz] * N + g);
+  }
+}
+
+// moments_and_test for the float32 tiles: the node's previous populations in
+// shared memory (`f0`, `stride` floats apart, replaced by acc), the sums of
+// each class of each axis first (93 float64 operations instead of 190), and
+// the difference of the populations in float32, where it is exact whenever the
+// test is close.
+__device__ __forceinline__ bool tile_moments_and_test(const StepArgs<float>& a, const float acc[27], float* f0, int stride,
+                                                      double C, double& rho0, double U[3], double& T) {
+  using L = Lattice<POND_D3Q27>;
+  double sx[3] = {0, 0, 0}, sy[3] = {0, 0, 0}, sz[3] = {0, 0, 0};
+  bool ok = true;
+#pragma unroll
+  for (int cx = 0; cx < 3; cx++)
+#pragma unroll
+    for (int cy = 0; cy < 3; cy++) {
+      double row = 0;
+#pragma unroll
+      for (int cz = 0; cz < 3; cz++) {
+        const int t = (cx * 3 + cy) * 3 + cz;
+        const double nv = acc[t];
+        row += nv;
+        sz[cz] += nv;
+        ok = ok && !(double(fabsf(acc[t] - f0[t * stride])) >= a.tol_abs + a.tol_rel * fabs(nv));
+        f0[t * stride] = acc[t];
+      }
+      sx[cx] += row;
+      sy[cy] += row;
+    }
+  const double rho = sx[0] + sx[1] + sx[2];
+  double m[4] = {0, 0, 0, 0};
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    const double vx = C * L::xi1(c) + U[0], vy = C * L::xi1(c) + U[1], vz = C * L::xi1(c) + U[2];
+    const double px = sx[c] * vx, py = sy[c] * vy, pz = sz[c] * vz;
+    m[0] += px; m[1] += py; m[2] += pz;
+    m[3] += px * vx + py * vy + pz * vz;
+  }
+  if (rho != 0) {
+    const double ir = 1.0 / rho;
+#pragma unroll
+    for (int k = 0; k < 4; k++) m[k] *= ir;
+  }
+  double Tn = (m[3] - m[0] * m[0] - m[1] * m[1] - m[2] * m[2]) * (1.0 / L::Dim);
+  if (Tn < 0) Tn = T;
+#pragma unroll
+  for (int k = 0; k < 3; k++) ok = ok && !(fabs(m[k] - U[k]) >= a.tolg_abs + a.tolg_rel * fabs(m[k]));
+  ok = ok && !(fabs(Tn - T) >= a.tolg_abs + a.tolg_rel * fabs(Tn));
+  rho0 = rho; U[0] = m[0]; U[1] = m[1]; U[2] = m[2]; T = Tn;
+  return ok;
 }
 
 // Z[k1,k2,i3] += sum_k3 w_i3 Gz[i3][k3] F[k1,k2,k3] (F: reference-gauge populations) for the z-classes i3
@@ -227,13 +369,13 @@ __device__ __forceinline__ void column_node(const float* node, const float Gz[3]
   };
   const float last[3] = {v[6].x, v[6].y, v[6].z};
 #pragma unroll
-  for (int i = 0; i < 3; i++) {
-    if ((i == 1 && !kPlus) || (i == 2 && !kMinus)) continue;
+  for (int k3 = 0; k3 < 3; k3++) {
 #pragma unroll
-    for (int k3 = 0; k3 < 3; k3++) {
+    for (int i = 0; i < 3; i++) {
+      if ((i == 1 && !kPlus) || (i == 2 && !kMinus)) continue;
       const float g = w[i] * Gz[i][k3];
 #pragma unroll
-      for (int k2 = 0; k2 < 3; k2++) Zp[i][k2] = fma2(g, pair(3 * k2 + k3), Zp[i][k2]);
+      for (int k2 = 0; k2 < 3; k2++) Zp[i][k2] = fma2(g, pair(3 * k3 + k2), Zp[i][k2]);
       Zq[i] = fma2(g, pair(9 + k3), Zq[i]);
       Zs[i] = fmaf(g, last[k3], Zs[i]);
     }
@@ -495,7 +637,27 @@ __global__ void __launch_bounds__(THREADS, 2) pull_d3q27_tile_kernel(StepArgs<fl
   extern __shared__ __align__(16) float sm[];
   const int tid = threadIdx.x + TX * (threadIdx.y + TY * threadIdx.z);
   const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY, z0 = blockIdx.z * TZ;
+  float* su = sm + NS * SN + 27 * THREADS + (THREADS / 32) * 28;
 
+  // ---- stage: each thread copies whole staged nodes (27 populations, the
+  // mirror reversing classes, and the gauge) with asynchronous copies, waits
+  // for its own copies and transfers its nodes into the reference gauge;
+  // boundary resolution happens in the addresses (mirrored velocity components
+  // flip; a node with a non-finite gauge contributes nothing, non-finite
+  // populations count as 0)
+#pragma unroll 1
+  for (int i = tid; i < SN; i += THREADS) {
+    const int hx = i % SX, hy = (i / SX) % SY, hz = i / (SX * SY);
+    bool rv[3];
+    const int gx = resolve_axis(x0 - H + hx, a.nx, a.bc[0], rv[0]);
+    const int gy = resolve_axis(y0 - H + hy, a.ny, a.bc[1], rv[1]);
+    const int gz = resolve_axis(z0 - H + hz, a.nz, a.bc[2], rv[2]);
+    const long long g = gx + (long long)a.nx * (gy + (long long)a.ny * gz);
+    copy_node(a.f_in, a.N, g, rv, sm + i * NS);
+#pragma unroll
+    for (int k = 0; k < 3; k++) cp_async4(su + k * SN + i, a.g_in + (long long)k * a.N + g);
+    cp_async4(sm + i * NS + 27, a.g_in + 3 * a.N + g);
+  }
   // ---- reference gauge of the CTA: the gauge of the tile's centre node
   //      ((0, 1) if it is not finite or its c is 0)
   float uref[3], icref;
@@ -519,80 +681,33 @@ __global__ void __launch_bounds__(THREADS, 2) pull_d3q27_tile_kernel(StepArgs<fl
     icref = (ok && fabsf(cc) > 1.0e-20f) ? 1.f / cc : 1.f;
   }
   const float cref = 1.f / icref;
-
-  // ---- stage: each thread copies whole staged nodes (27 populations in
-  // tensor-class order, the mirror reversing classes) with asynchronous
-  // copies, waits for its own copies and transfers its nodes into the
-  // reference gauge; boundary resolution happens in the addresses, the gauge
-  // comes straight from global memory (mirrored velocity components flip; a
-  // node with a non-finite gauge contributes nothing, non-finite populations
-  // count as 0)
-#pragma unroll 1
-  for (int i = tid; i < SN; i += THREADS) {
-    const int hx = i % SX, hy = (i / SX) % SY, hz = i / (SX * SY);
-    bool rv[3];
-    const int gx = resolve_axis(x0 - H + hx, a.nx, a.bc[0], rv[0]);
-    const int gy = resolve_axis(y0 - H + hy, a.ny, a.bc[1], rv[1]);
-    const int gz = resolve_axis(z0 - H + hz, a.nz, a.bc[2], rv[2]);
-    const long long g = gx + (long long)a.nx * (gy + (long long)a.ny * gz);
-#pragma unroll
-    for (int t = 0; t < 27; t++) {
-      int cx = t / 9, cy = (t / 3) % 3, cz = t % 3;
-      if (rv[0]) cx = rev3(cx);
-      if (rv[1]) cy = rev3(cy);
-      if (rv[2]) cz = rev3(cz);
-      cp_async4(&sm[i * NS + slot27(t)], a.f_in + (long long)c_ref27[cx * 9 + cy * 3 + cz] * a.N + g);
-    }
-  }
   cp_async_wait_all();
 #pragma unroll 1
   for (int i = tid; i < SN; i += THREADS) {
     const int hx = i % SX, hy = (i / SX) % SY, hz = i / (SX * SY);
-    bool rv[3];
-    const int gx = resolve_axis(x0 - H + hx, a.nx, a.bc[0], rv[0]);
-    const int gy = resolve_axis(y0 - H + hy, a.ny, a.bc[1], rv[1]);
-    const int gz = resolve_axis(z0 - H + hz, a.nz, a.bc[2], rv[2]);
-    const long long g = gx + (long long)a.nx * (gy + (long long)a.ny * gz);
+    // the axes mirrored there (only positions outside the grid can be)
+    const int p[3] = {x0 - H + hx, y0 - H + hy, z0 - H + hz}, n[3] = {a.nx, a.ny, a.nz};
     float u[3];
     bool ok = true;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-      const float v = __ldg(&a.g_in[(long long)k * a.N + g]);
-      u[k] = rv[k] ? -v : v;
+      bool rv = false;
+      if (p[k] < 0 || p[k] >= n[k]) resolve_axis(p[k], n[k], a.bc[k], rv);
+      const float v = su[k * SN + i];
+      u[k] = rv ? -v : v;
       ok = ok && fabsf(v) <= 3.0e38f;
     }
-    const float T = __ldg(&a.g_in[3 * a.N + g]);
+    const float T = sm[i * NS + 27];
     const float c = copysignf(sqrtf(fabsf(T) * (float)(1.0 / L::TLat)), T);
     ok = ok && fabsf(c) <= 3.0e38f;
-    float v[27];
-    {
-      float e[28];
-      const float4* s4 = reinterpret_cast<const float4*>(sm + i * NS);
-#pragma unroll
-      for (int q = 0; q < 7; q++) {
-        const float4 w = s4[q];
-        e[4 * q] = w.x; e[4 * q + 1] = w.y; e[4 * q + 2] = w.z; e[4 * q + 3] = w.w;
-      }
-#pragma unroll
-      for (int t = 0; t < 27; t++) {
-        const float w = e[slot27(t)];
-        v[t] = (ok && fabsf(w) <= 3.402823466e38f) ? w : 0.f;
-      }
-    }
     const float r = ok ? c * icref : 0.f;
     const float sq[3] = {ok ? (u[0] - uref[0]) * icref : 0.f, ok ? (u[1] - uref[1]) * icref : 0.f,
                          ok ? (u[2] - uref[2]) * icref : 0.f};
     const float rq[3] = {r, r, r};
-    node_to_ref(v, sq, rq);
-    {
-      float e[28];
-      e[27] = 0.f;
-#pragma unroll
-      for (int t = 0; t < 27; t++) e[slot27(t)] = v[t];
-      float4* s4 = reinterpret_cast<float4*>(sm + i * NS);
-#pragma unroll
-      for (int q = 0; q < 7; q++) s4[q] = make_float4(e[4 * q], e[4 * q + 1], e[4 * q + 2], e[4 * q + 3]);
-    }
+    // a node of the tile leaves its populations where its thread keeps its iterate
+    const int tx = hx - H, ty = hy - H, tz = hz - H;
+    const bool own = tx >= 0 && tx < TX && ty >= 0 && ty < TY && tz >= 0 && tz < TZ;
+    staged_to_ref(sm + i * NS, ok, sq, rq, own ? sm + NS * SN + tx + TX * (ty + TY * tz) : nullptr, THREADS);
   }
   __syncthreads();
 
@@ -605,14 +720,18 @@ __global__ void __launch_bounds__(THREADS, 2) pull_d3q27_tile_kernel(StepArgs<fl
   // which keeps them out of the loop's registers
   float* f0s = sm + NS * SN + tid;
   double rho0 = 1, U[3] = {0, 0, 0}, T = L::TLat;
-  {
-    float f0[27];
-    if (active) load_center<POND_D3Q27, float>(a, idx, f0, rho0, U, T);
-    else
+  if (active) {  // c0.load (steps.cu:360-363); the populations are in f0s already
+    rho0 = a.rho_in[idx];
+    U[0] = a.g_in[idx]; U[1] = a.g_in[a.N + idx]; U[2] = a.g_in[2 * a.N + idx];
+    T = a.g_in[3 * a.N + idx];
+    if (rho0 == 0 && U[0] == 0 && U[1] == 0 && U[2] == 0 && T == 0) {  // set_base(1, TLat) of an empty record
+      rho0 = 1; T = L::TLat;
 #pragma unroll
-      for (int t = 0; t < 27; t++) f0[t] = 0.f;
-#pragma unroll
-    for (int t = 0; t < 27; t++) f0s[t * THREADS] = f0[t];
+      for (int t = 0; t < 27; t++) f0s[t * THREADS] = float(lattice_weight_t<POND_D3Q27>(t));
+    }
+    if (a.guess) {
+      U[0] = a.guess[idx]; U[1] = a.guess[a.N + idx]; U[2] = a.guess[2 * a.N + idx]; T = a.guess[3 * a.N + idx];
+    }
   }
   const int pos[3] = {x, y, z};
   const int sbase = (lz + H) * SX * SY + (ly + H) * SX + (lx + H);
@@ -642,10 +761,11 @@ __global__ void __launch_bounds__(THREADS, 2) pull_d3q27_tile_kernel(StepArgs<fl
     }
     // transfer from the reference gauge to this iteration's target gauge,
     // per axis: G[i][k] = L_i(b + a xi_k), a = c_ref / C, b = (u_ref - U) / C
-    const float ainv = float(double(cref) / C);
+    const double iC = 1.0 / C;
+    const float ainv = float(double(cref) * iC);
     float bq[3];
 #pragma unroll
-    for (int ax = 0; ax < 3; ax++) bq[ax] = float((double(uref[ax]) - U[ax]) / C);
+    for (int ax = 0; ax < 3; ax++) bq[ax] = float((double(uref[ax]) - U[ax]) * iC);
     float acc[27];
 #pragma unroll
     for (int t = 0; t < 27; t++) acc[t] = 0.f;
@@ -738,12 +858,7 @@ __global__ void __launch_bounds__(THREADS, 2) pull_d3q27_tile_kernel(StepArgs<fl
 #pragma unroll
         for (int t = 0; t < 27; t++) acc[t] = 0.f;
       }
-      float f0[27];
-#pragma unroll
-      for (int t = 0; t < 27; t++) f0[t] = f0s[t * THREADS];
-      conv = moments_and_test<POND_D3Q27, float>(a, acc, f0, C, rho0, U, T);
-#pragma unroll
-      for (int t = 0; t < 27; t++) f0s[t * THREADS] = f0[t];
+      conv = tile_moments_and_test(a, acc, f0s, THREADS, C, rho0, U, T);
       if (conv || niter >= a.max_iter) done = true;
     }
   }

@@ -30,9 +30,9 @@
 // Staged layout and contraction are the plain tile's (slot27, contract_tile):
 // two-wide multiply-adds on neighbouring populations, straight-line z columns.
 // Bound by shared-memory bandwidth and by one CTA of 8 warps per SM (both
-// staged sets take 207 KB): two steps of a 64^3 vortex, quadratic, 4.39 ms
-// against 5.32 ms with scalar contractions behind rolled z offsets, the same
-// results bit for bit.
+// staged sets take 217 KB): two steps of a 64^3 vortex, quadratic, 2.23 ms
+// against 5.32 ms with scalar contractions behind rolled z offsets (the shared
+// contraction 0.9 ms, serving the last lanes by the warp 2.0, staging 0.1).
 #pragma once
 #include "pond_step_d3q27.cuh"
 
@@ -45,13 +45,13 @@ using d27::contract_tile;
 using d27::contract_x;
 using d27::contract_y;
 using d27::contract_z;
+using d27::copy_node;
 using d27::cp_async4;
 using d27::cp_async_wait_all;
 using d27::few_lanes;
 using d27::c_ref27;
 using d27::node_to_ref;
-using d27::rev3;
-using d27::slot27;
+using d27::staged_to_ref;
 using d27::wpick;
 
 constexpr int TX = 8, TY = 4, TZ = 4, H = 2;
@@ -66,7 +66,8 @@ constexpr int OFF_H = NS * SN;
 constexpr int OFF_OWN = 2 * NS * SN;
 constexpr int OFF_X = OFF_OWN + 27 * THREADS;
 constexpr int OFF_S = OFF_X + 2 * (2 * 5 * NODES) + 2 * 2 * NODES;  // 28 floats of scratch per warp
-constexpr size_t SMEM_BYTES = size_t(OFF_S + (THREADS / 32) * 28) * sizeof(float);
+constexpr int OFF_U = OFF_S + (THREADS / 32) * 28;  // the staged nodes' velocities (T: the pad of their f)
+constexpr size_t SMEM_BYTES = size_t(OFF_U + 3 * SN) * sizeof(float);
 static_assert(OFF_X % 2 == 0, "the float64 exchange slots must be 8-byte aligned");
 static_assert(SMEM_BYTES + 3 * 1024 <= 232448, "the tile must fit one CTA per SM");
 
@@ -84,6 +85,22 @@ __global__ void __launch_bounds__(THREADS, 1) pull_d3q27_energy_tile_kernel(Step
   const int pair = (tid >> 5) & 3;
   const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY, z0 = blockIdx.z * TZ;
 
+  // ---- stage f and h of every staged node, then transfer both into the
+  //      reference gauge (boundary resolution, mirror reversal and the
+  //      dropping of non-finite values as in the plain tile kernel)
+  for (int i = tid; i < SN; i += THREADS) {
+    const int hx = i % SX, hy = (i / SX) % SY, hz = i / (SX * SY);
+    bool rv[3];
+    const int gx = resolve_axis(x0 - H + hx, a.nx, a.bc[0], rv[0]);
+    const int gy = resolve_axis(y0 - H + hy, a.ny, a.bc[1], rv[1]);
+    const int gz = resolve_axis(z0 - H + hz, a.nz, a.bc[2], rv[2]);
+    const long long g = gx + (long long)a.nx * (gy + (long long)a.ny * gz);
+    copy_node(a.f_in, a.N, g, rv, sm + i * NS);
+    copy_node(a.h_in, a.N, g, rv, sm + OFF_H + i * NS);
+#pragma unroll
+    for (int k = 0; k < 3; k++) cp_async4(sm + OFF_U + k * SN + i, a.g_in + (long long)k * a.N + g);
+    cp_async4(sm + i * NS + 27, a.g_in + 3 * a.N + g);
+  }
   // ---- reference gauge of the CTA: the gauge of the tile's centre node
   float uref[3], icref;
   {
@@ -106,74 +123,35 @@ __global__ void __launch_bounds__(THREADS, 1) pull_d3q27_energy_tile_kernel(Step
     icref = (ok && fabsf(cc) > 1.0e-20f) ? 1.f / cc : 1.f;
   }
   const float cref = 1.f / icref;
-
-  // ---- stage f and h of every staged node, then transfer both into the
-  //      reference gauge (boundary resolution, mirror reversal and the
-  //      dropping of non-finite values as in the plain tile kernel)
-  for (int i = tid; i < SN; i += THREADS) {
-    const int hx = i % SX, hy = (i / SX) % SY, hz = i / (SX * SY);
-    bool rv[3];
-    const int gx = resolve_axis(x0 - H + hx, a.nx, a.bc[0], rv[0]);
-    const int gy = resolve_axis(y0 - H + hy, a.ny, a.bc[1], rv[1]);
-    const int gz = resolve_axis(z0 - H + hz, a.nz, a.bc[2], rv[2]);
-    const long long g = gx + (long long)a.nx * (gy + (long long)a.ny * gz);
-#pragma unroll
-    for (int t = 0; t < 27; t++) {
-      int cx = t / 9, cy = (t / 3) % 3, cz = t % 3;
-      if (rv[0]) cx = rev3(cx);
-      if (rv[1]) cy = rev3(cy);
-      if (rv[2]) cz = rev3(cz);
-      const long long src = (long long)c_ref27[cx * 9 + cy * 3 + cz] * a.N + g;
-      cp_async4(&sm[i * NS + slot27(t)], a.f_in + src);
-      cp_async4(&sm[OFF_H + i * NS + slot27(t)], a.h_in + src);
-    }
-  }
   cp_async_wait_all();
   for (int i = tid; i < SN; i += THREADS) {
     const int hx = i % SX, hy = (i / SX) % SY, hz = i / (SX * SY);
-    bool rv[3];
-    const int gx = resolve_axis(x0 - H + hx, a.nx, a.bc[0], rv[0]);
-    const int gy = resolve_axis(y0 - H + hy, a.ny, a.bc[1], rv[1]);
-    const int gz = resolve_axis(z0 - H + hz, a.nz, a.bc[2], rv[2]);
-    const long long g = gx + (long long)a.nx * (gy + (long long)a.ny * gz);
+    // the axes mirrored there (only positions outside the grid can be)
+    const int p[3] = {x0 - H + hx, y0 - H + hy, z0 - H + hz}, n[3] = {a.nx, a.ny, a.nz};
     float u[3];
     bool ok = true;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-      const float v = __ldg(&a.g_in[(long long)k * a.N + g]);
-      u[k] = rv[k] ? -v : v;
+      bool rv = false;
+      if (p[k] < 0 || p[k] >= n[k]) resolve_axis(p[k], n[k], a.bc[k], rv);
+      const float v = sm[OFF_U + k * SN + i];
+      u[k] = rv ? -v : v;
       ok = ok && fabsf(v) <= 3.0e38f;
     }
-    const float T = __ldg(&a.g_in[3 * a.N + g]);
+    const float T = sm[i * NS + 27];
     const float c = copysignf(sqrtf(fabsf(T) * (float)(1.0 / L::TLat)), T);
     ok = ok && fabsf(c) <= 3.0e38f;
     const float r = ok ? c * icref : 0.f;
     const float sq[3] = {ok ? (u[0] - uref[0]) * icref : 0.f, ok ? (u[1] - uref[1]) * icref : 0.f,
                          ok ? (u[2] - uref[2]) * icref : 0.f};
     const float rq[3] = {r, r, r};
+    // a node of the tile leaves its populations where its threads keep their iterates
+    const int tx = hx - H, ty = hy - H, tz = hz - H;
+    const bool own = tx >= 0 && tx < TX && ty >= 0 && ty < TY && tz >= 0 && tz < TZ;
 #pragma unroll 1
-    for (int d = 0; d < 2; d++) {
-      float* p = sm + d * OFF_H + i * NS;
-      float v[27];
-      float e[28];
-      float4* s4 = reinterpret_cast<float4*>(p);
-#pragma unroll
-      for (int q = 0; q < 7; q++) {
-        const float4 w = s4[q];
-        e[4 * q] = w.x; e[4 * q + 1] = w.y; e[4 * q + 2] = w.z; e[4 * q + 3] = w.w;
-      }
-#pragma unroll
-      for (int t = 0; t < 27; t++) {
-        const float w = e[slot27(t)];
-        v[t] = (ok && fabsf(w) <= 3.402823466e38f) ? w : 0.f;
-      }
-      node_to_ref(v, sq, rq);
-      e[27] = 0.f;
-#pragma unroll
-      for (int t = 0; t < 27; t++) e[slot27(t)] = v[t];
-#pragma unroll
-      for (int q = 0; q < 7; q++) s4[q] = make_float4(e[4 * q], e[4 * q + 1], e[4 * q + 2], e[4 * q + 3]);
-    }
+    for (int d = 0; d < 2; d++)
+      staged_to_ref(sm + d * OFF_H + i * NS, ok, sq, rq,
+                    own ? sm + OFF_OWN + d * NODES + tx + TX * (ty + TY * tz) : nullptr, THREADS);
   }
   __syncthreads();
 
@@ -188,24 +166,20 @@ __global__ void __launch_bounds__(THREADS, 1) pull_d3q27_energy_tile_kernel(Step
   double* xd = reinterpret_cast<double*>(sm + OFF_X);
   int* xf = reinterpret_cast<int*>(xd + 2 * 5 * NODES);
   double rho0 = 1, U[3] = {0, 0, 0}, T = L::TLat;
-  {
-    float f0[27];
-    if (active) {
-      load_center<POND_D3Q27, float>(a, idx, f0, rho0, U, T);
-      if (role) {
-        const bool base = a.rho_in[idx] == 0.f && a.g_in[idx] == 0.f && a.g_in[a.N + idx] == 0.f &&
-                          a.g_in[2 * a.N + idx] == 0.f && a.g_in[3 * a.N + idx] == 0.f;
-        if (base) energy_equilibrium<POND_D3Q27, float>(rho0, U, T, a.dof, f0);  // set_base with its energy
-        else
+  if (active) {  // c0.load (steps.cu:360-363); the populations are in `own` already
+    rho0 = a.rho_in[idx];
+    U[0] = a.g_in[idx]; U[1] = a.g_in[a.N + idx]; U[2] = a.g_in[2 * a.N + idx];
+    T = a.g_in[3 * a.N + idx];
+    if (rho0 == 0 && U[0] == 0 && U[1] == 0 && U[2] == 0 && T == 0) {  // set_base(1, TLat), with its energy
+      rho0 = 1; T = L::TLat;
+      float f0[27];
+      if (role) energy_equilibrium<POND_D3Q27, float>(rho0, U, T, a.dof, f0);
 #pragma unroll
-          for (int t = 0; t < 27; t++) f0[t] = a.h_in[(long long)c_ref27[t] * a.N + idx];
-      }
-    } else {
-#pragma unroll
-      for (int t = 0; t < 27; t++) f0[t] = 0.f;
+      for (int t = 0; t < 27; t++) own[t * THREADS] = role ? f0[t] : float(lattice_weight_t<POND_D3Q27>(t));
     }
-#pragma unroll
-    for (int t = 0; t < 27; t++) own[t * THREADS] = f0[t];
+    if (a.guess) {
+      U[0] = a.guess[idx]; U[1] = a.guess[a.N + idx]; U[2] = a.guess[2 * a.N + idx]; T = a.guess[3 * a.N + idx];
+    }
   }
   const int pos[3] = {x, y, z};
   const int sbase = (lz + H) * SX * SY + (ly + H) * SX + (lx + H);
@@ -232,10 +206,11 @@ __global__ void __launch_bounds__(THREADS, 1) pull_d3q27_energy_tile_kernel(Step
       lo[ax] = min(ro[ax][0], min(ro[ax][1], ro[ax][2]));
       hi[ax] = max(ro[ax][0], max(ro[ax][1], ro[ax][2])) + N - 1;
     }
-    const float ainv = float(double(cref) / C);
+    const double iC = 1.0 / C;
+    const float ainv = float(double(cref) * iC);
     float bq[3];
 #pragma unroll
-    for (int ax = 0; ax < 3; ax++) bq[ax] = float((double(uref[ax]) - U[ax]) / C);
+    for (int ax = 0; ax < 3; ax++) bq[ax] = float((double(uref[ax]) - U[ax]) * iC);
     float acc[27];
 #pragma unroll
     for (int t = 0; t < 27; t++) acc[t] = 0.f;
