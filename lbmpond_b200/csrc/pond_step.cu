@@ -202,14 +202,34 @@ template <int LAT, int N, typename R> static void launch_point(const StepArgs<R>
 // (4M nodes: 0.51 ms, 0.73 ms looped).
 static int gap2_ctas(int nx) { return (nx + 127) / 128 < 148 * 6 ? (nx + 127) / 128 : 148 * 6; }
 
+// Launch a step kernel that may start while the step before it on the stream
+// runs its last CTAs; it waits in the kernel for that step to complete
+// (cudaGridDependencySynchronize).  Hides the launch of every step but the
+// first: 1000 nodes of D1Q5 9.2 us per step instead of 10.3.
+template <typename R>
+static cudaError_t launch_early(void (*kern)(StepArgs<R>), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                                const StepArgs<R>& a) {
+  cudaLaunchAttribute early;
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &early;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, a);
+}
+
 // D1Q5, one step of a 1D grid of at most W1D_MAX nodes with a warp per node:
 // there the step is one node's chain of iterations, however many nodes; above
 // it the one-thread-per-node kernels do more nodes per instruction.  Measured,
 // us per step, warp / thread per node (TVD float64, WENO5 float32, cubic
-// float32): 1000 nodes 10.3 / 32.4, 10.4 / 26.7, 8.6 / 14.4; 4000 nodes 17.0 /
-// 32.1, 20.6 / 26.7, 13.7 / 14.4; 8000 nodes 27.5 / 33.1, 35.0 / 26.7, 19.3 / 14.4.
+// float32): 1000 nodes 9.1 / 32.4, 9.8 / 26.7, 7.6 / 14.4; 4000 nodes 15.1 /
+// 32.1, 18.7 / 26.7, 12.3 / 14.4; 8000 nodes about 27 / 33, 34 / 27, 19 / 14.
 static constexpr int W1D_MAX = 4096;
-template <typename R> static bool launch_1d_warp(const StepArgs<R>& a, int interp, cudaStream_t s) {
+template <typename R> static bool launch_1d_warp(const StepArgs<R>& a, int interp, cudaStream_t s, cudaError_t& e) {
   if (a.nx > W1D_MAX || a.ny != 1 || a.nz != 1) return false;
   void (*kern)(StepArgs<R>) = nullptr;
   switch (interp) {
@@ -222,7 +242,7 @@ template <typename R> static bool launch_1d_warp(const StepArgs<R>& a, int inter
     case POND_WENO5_ROW: kern = w1d::pull_1d_warp_kernel<POND_WENO5, R>; break;
     default: return false;  // the mesh schemes
   }
-  kern<<<(a.nx + w1d::WARPS - 1) / w1d::WARPS, w1d::THREADS, 0, s>>>(a);
+  e = launch_early(kern, dim3((a.nx + w1d::WARPS - 1) / w1d::WARPS), dim3(w1d::THREADS), 0, s, a);
   return true;
 }
 
@@ -355,7 +375,10 @@ template <typename R> static int launch_typed(pond_ctx* c, const void* const* in
   }
   switch (c->p.lattice) {
     case POND_D1Q5:
-      if (launch_1d_warp<R>(a, c->p.interp, s)) break;
+      if (launch_1d_warp<R>(a, c->p.interp, s, e)) {
+        if (e != cudaSuccess) return cuda_fail(e, "step kernel launch");
+        break;
+      }
       switch (c->p.interp) {
         case POND_LAGR2: launch_point<POND_D1Q5, 2, R>(a, s); break;
         case POND_LAGR3: launch_point<POND_D1Q5, 3, R>(a, s); break;
@@ -387,7 +410,8 @@ template <typename R> static int launch_typed(pond_ctx* c, const void* const* in
                                                                       : d27::pull_d3q27_tile_kernel<4>;
           e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d27::SMEM_BYTES);
           if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute");
-          kern<<<grd, blk, d27::SMEM_BYTES, s>>>(a);
+          e = launch_early(kern, grd, blk, d27::SMEM_BYTES, s, a);
+          if (e != cudaSuccess) return cuda_fail(e, "step kernel launch");
           break;
         }
       } else if (c->p.interp >= POND_LAGR2 && c->p.interp <= POND_LAGR4) {

@@ -9,9 +9,9 @@
 //
 // What bounds it: the dependent chain of an iteration (square root, window,
 // transfer, limiter, moments, reciprocal; float64 throughout for TVD and
-// WENO5's nonlinear part), about 1 us, and the launch, first loads and
-// reductions of a step, about 5 us.  1000 nodes, TVD, float64, 3.6 iterations:
-// 10.3 us per step against 32.4 us with a thread per node, whose iteration
+// WENO5's nonlinear part), about 1 us, and the first loads and reductions of a
+// step, about 4 us.  1000 nodes, TVD, float64, 3.6 iterations: 9.1 us per step
+// against 32.4 us with a thread per node, whose iteration
 // transfers six nodes by five populations and selects 80 weights in one chain.
 #pragma once
 #include "pond_step_1d.cuh"
@@ -61,6 +61,10 @@ template <int SCHEME, typename R> __global__ void __launch_bounds__(THREADS) pul
   const int k = min(lane / LANES, 4), e = lane < 30 ? lane % LANES : lane - 30;  // lanes 30, 31 repeat population 4
   const int x = blockIdx.x * WARPS + warp;
   NodeSums ns = {0, 0, 0, 0, 0, 0, 0ull, 0ull, 0ull, 0};
+  // launched while the step before still runs (launch_1d_warp): let the next
+  // one come, then wait for the step before to be complete and visible
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
   if (x < a.nx) {  // warp-uniform
     R f0[5];
     double rho0, U[3], T;

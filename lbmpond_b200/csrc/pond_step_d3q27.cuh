@@ -574,8 +574,9 @@ __device__ __forceinline__ void contract_live_lanes(unsigned live, const float* 
 }
 
 // Live lanes at which the warp serves nodes one by one: the serial iteration
-// costs about 11,000 / 6,500 / 3,000 instructions (N = 4 / 3 / 2), a node by the warp 1,200.
-template <int N> __host__ __device__ constexpr int few_lanes() { return N == 4 ? 5 : N == 3 ? 3 : 1; }
+// costs about 11,000 / 6,500 / 3,000 instructions (N = 4 / 3 / 2), a node by
+// the warp 1,200.  8 / 5 / 2 lanes measured 0.4-1.5 % faster than 5 / 3 / 1.
+template <int N> __host__ __device__ constexpr int few_lanes() { return N == 4 ? 8 : N == 3 ? 5 : 2; }
 
 // Partial record of the step sums, updated instead of the context's sums
 // when the kernel runs without a context (kPartials = true; a.sums then
@@ -638,6 +639,10 @@ __global__ void __launch_bounds__(THREADS, 2) pull_d3q27_tile_kernel(StepArgs<fl
   const int tid = threadIdx.x + TX * (threadIdx.y + TY * threadIdx.z);
   const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY, z0 = blockIdx.z * TZ;
   float* su = sm + NS * SN + 27 * THREADS + (THREADS / 32) * 28;
+  // launched while the step before still runs (launch_early): let the next one
+  // come, then wait for the step before to be complete and visible
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
 
   // ---- stage: each thread copies whole staged nodes (27 populations, the
   // mirror reversing classes, and the gauge) with asynchronous copies, waits
