@@ -426,6 +426,10 @@ template <int SCHEME, int NT>
 __global__ void __launch_bounds__(NT, 1) batch_kernel(Args a) {
   using L = Lattice<POND_D1Q5>;
   constexpr int GROUP = SCHEME == POND_WENO5 ? 5 : 4;  // lanes per population in phase 2
+  // at 64 registers a thread pull_near's 35 transferred values spill, which
+  // costs the general way more (log-uniform tubes, 1000 steps: 4.46 against
+  // 3.8 ms per step) than the near way gains there
+  constexpr bool NEAR_FITS = NT <= 768;
   extern __shared__ __align__(16) float sm[];
   float* sf = sm;                // [5][BIN_CAP]
   float* su = sm + 5 * BIN_CAP;  // u
@@ -464,7 +468,7 @@ __global__ void __launch_bounds__(NT, 1) batch_kernel(Args a) {
         bulk_g2s(su, a.u + off, bytes, &s_bar);
         bulk_g2s(sT, a.T + off, bytes, &s_bar);
       }
-      const bool count_hot = step % HOT_EVERY == 0;
+      const bool count_hot = NEAR_FITS && step % HOT_EVERY == 0;
       if (count_hot && tid < BIN_SEGS) s_hot[tid] = 0;
       const bool staged = mbar_wait(&s_bar, phase & 1u);
       phase++;
@@ -518,7 +522,9 @@ __global__ void __launch_bounds__(NT, 1) batch_kernel(Args a) {
         float fn[5];
 #pragma unroll
         for (int k = 0; k < 5; k++) vk[k] = C * L::xi1(k) + s.U;
-        if (!cold || !pull_near<SCHEME>(sf, su, sc, ps, n, s.x - ps, vk, Uf, invC, fn))
+        bool near = false;
+        if constexpr (NEAR_FITS) near = cold && pull_near<SCHEME>(sf, su, sc, ps, n, s.x - ps, vk, Uf, invC, fn);
+        if (!near)
 #pragma unroll
           for (int k = 0; k < 5; k++) fn[k] = pull_population<SCHEME>(k, sf, su, sc, ps, n, s.x - ps, vk[k], Uf, invC);
         const bool ok = moments_and_test(a, fn, vk, s);

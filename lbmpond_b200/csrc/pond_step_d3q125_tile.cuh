@@ -1,14 +1,15 @@
-// D3Q125 PonD pull step, float32 or float64: a tile of nodes per CTA, a warp
-// per node.
+// D3Q125 PonD pull step in float64, and with energy populations in float32 or
+// float64: a tile of nodes per CTA, a warp per node.  (The plain float32 step
+// is pond_step_d3q125_rows.cuh, whose tile has no room for either.)
 //
 // The arithmetic of steps.cu:151-250 PonDstepD3Q125 (quadratic stencil with
 // its origin fixed at coord-1, gauge transfer by the 5-point Lagrange basis,
 // float64 moments and convergence test), organised for the SM:
 //
 //  * a CTA owns a 4 x 4 x 4 tile and stages it with its +-1 halo (6 x 6 x 6
-//    nodes: 125 population planes, the gauge velocities and c, 113 KB) once
-//    per step, so two CTAs fit on an SM and every staged node serves up to
-//    27 centres from shared memory;
+//    nodes: 125 population planes, the gauge velocities and c; 113 KB of
+//    float32 and population set) once per step, so every staged node serves up
+//    to 27 centres from shared memory;
 //  * after staging, one thread per staged node transfers its populations
 //    into a reference gauge R shared by the CTA (the gauge of a tile node):
 //    three passes of the 5x5 basis.  The transfer of a source node into a
@@ -55,9 +56,7 @@ template <bool kE, typename Rs = float, int TT = T> struct SmemT {
   unsigned char flags[SNT]; // mirrored axes (bits 0-2)
   Rs GY[WARPS][3][25];      // per warp and iteration: y weight x transfer entry, [n_y][5 i2 + k2]
 };
-using Smem = SmemT<false>;
 
-static_assert(2 * (sizeof(SmemT<false>) + 1024) <= 233472, "two CTAs must fit in the 228 KB of an SM");
 static_assert(sizeof(SmemT<true>) + 1024 <= 233472, "the energy variant must fit one CTA per SM");
 static_assert(sizeof(SmemT<false, double>) <= 232448, "the float64 tile must fit one CTA");
 static_assert(sizeof(SmemT<true, double, 2>) <= 232448, "the float64 energy tile must fit one CTA");
@@ -122,7 +121,7 @@ __device__ __forceinline__ void stencil_weights(int pos, double C, double U, int
 // R: storage and transfer type (float64: one CTA per SM).
 // TT: tile edge (2 for the float64 energy variant: 8 nodes, one per warp).
 template <bool kE, typename R = float, int TT = T>
-__global__ void __launch_bounds__(THREADS, (kE || sizeof(R) == 8) ? 1 : 2) pull_d3q125_tile_kernel(StepArgs<R> a) {
+__global__ void __launch_bounds__(THREADS, 1) pull_d3q125_tile_kernel(StepArgs<R> a) {
   static_assert(!(kE && sizeof(R) == 8 && TT > 2), "a float64 4^3 tile has no room for energy populations");
   constexpr int S = TT + 2, SN = S * S * S, PS = SN + 1;  // staged edge, staged nodes, plane stride
   using L = Lattice<POND_D3Q125>;
