@@ -100,6 +100,23 @@ static bool any_overlap(long long N, const float* fi, const float* ri, const flo
   return false;
 }
 
+template <int N> static dim3 grid(const StepArgs<float>& a) {
+  using Ti = d27::Tile<N>;
+  return dim3((a.nx + Ti::TX - 1) / Ti::TX, (a.ny + Ti::TY - 1) / Ti::TY, (a.nz + Ti::TZ - 1) / Ti::TZ);
+}
+template <int N> static long long ctas(const StepArgs<float>& a) {
+  const dim3 g = grid<N>(a);
+  return (long long)g.x * g.y * g.z;
+}
+template <int N> static void launch(const StepArgs<float>& a, cudaStream_t s) {
+  using Ti = d27::Tile<N>;
+  d27::pull_d3q27_tile_kernel<N, true><<<grid<N>(a), Ti::THREADS, Ti::SMEM_BYTES, s>>>(a);
+}
+template <int N> static cudaError_t opt_in() {
+  return cudaFuncSetAttribute(d27::pull_d3q27_tile_kernel<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)d27::Tile<N>::SMEM_BYTES);
+}
+
 // Once per device: the scratch array's device address and the step kernels'
 // shared-memory opt-in.  Called with the target device current.
 static int setup_device(void** addr) {
@@ -112,14 +129,9 @@ static int setup_device(void** addr) {
     void* p = nullptr;
     e = cudaGetSymbolAddress(&p, g_partials);
     if (e != cudaSuccess) return cuda_fail(e, "cudaGetSymbolAddress(scratch)");
-    e = cudaFuncSetAttribute(d27::pull_d3q27_tile_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)d27::SMEM_BYTES);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(d27::pull_d3q27_tile_kernel<3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)d27::SMEM_BYTES);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(d27::pull_d3q27_tile_kernel<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)d27::SMEM_BYTES);
+    e = opt_in<2>();
+    if (e == cudaSuccess) e = opt_in<3>();
+    if (e == cudaSuccess) e = opt_in<4>();
     if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute");
     g_partials_addr[dev] = p;
   }
@@ -177,16 +189,15 @@ extern "C" int pond_step_noalloc(const pond_params* p, const float* f_in, const 
   const double PI = 3.14159265358979323846;
   a.kdx = 0.5 / (8 * PI * PI * PI) * (2 * PI / p->Nx) * (2 * PI / p->Ny) * (2 * PI / p->Nz);
   cudaStream_t s = (cudaStream_t)stream;
-  const dim3 grd((unsigned)((p->Nx + d27::TX - 1) / d27::TX), (unsigned)((p->Ny + d27::TY - 1) / d27::TY),
-                 (unsigned)((p->Nz + d27::TZ - 1) / d27::TZ));
-  const dim3 blk(d27::TX, d27::TY, d27::TZ);
-  const long long ctas = (long long)grd.x * grd.y * grd.z;
+  const long long ctas = p->interp == POND_LAGR2   ? noalloc::ctas<2>(a)
+                         : p->interp == POND_LAGR3 ? noalloc::ctas<3>(a)
+                                                   : noalloc::ctas<4>(a);
   const int nrec = (int)(ctas < d27::PARTIALS ? ctas : d27::PARTIALS);
   cudaError_t e = cudaMemsetAsync(scratch, 0, (size_t)nrec * sizeof(d27::BlockPartial), s);
   if (e != cudaSuccess) return cuda_fail(e, "pond_step_noalloc scratch reset");
-  if (p->interp == POND_LAGR2) d27::pull_d3q27_tile_kernel<2, true><<<grd, blk, d27::SMEM_BYTES, s>>>(a);
-  else if (p->interp == POND_LAGR3) d27::pull_d3q27_tile_kernel<3, true><<<grd, blk, d27::SMEM_BYTES, s>>>(a);
-  else d27::pull_d3q27_tile_kernel<4, true><<<grd, blk, d27::SMEM_BYTES, s>>>(a);
+  if (p->interp == POND_LAGR2) noalloc::launch<2>(a, s);
+  else if (p->interp == POND_LAGR3) noalloc::launch<3>(a, s);
+  else noalloc::launch<4>(a, s);
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "pond_step_noalloc step launch");
   noalloc::reduce_partials_kernel<<<1, 256, 0, s>>>(reinterpret_cast<const d27::BlockPartial*>(scratch),

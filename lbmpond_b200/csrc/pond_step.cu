@@ -222,6 +222,15 @@ static cudaError_t launch_early(void (*kern)(StepArgs<R>), dim3 grid, dim3 block
   return cudaLaunchKernelEx(&cfg, kern, a);
 }
 
+template <int N> static cudaError_t launch_d3q27_tile(const StepArgs<float>& a, cudaStream_t s) {
+  using Ti = d27::Tile<N>;
+  const cudaError_t e = cudaFuncSetAttribute(d27::pull_d3q27_tile_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)Ti::SMEM_BYTES);
+  if (e != cudaSuccess) return e;
+  const dim3 grd((a.nx + Ti::TX - 1) / Ti::TX, (a.ny + Ti::TY - 1) / Ti::TY, (a.nz + Ti::TZ - 1) / Ti::TZ);
+  return launch_early(&d27::pull_d3q27_tile_kernel<N>, grd, dim3(Ti::THREADS), Ti::SMEM_BYTES, s, a);
+}
+
 // D1Q5, one step of a 1D grid of at most W1D_MAX nodes with a warp per node:
 // there the step is one node's chain of iterations, however many nodes; above
 // it the one-thread-per-node kernels do more nodes per instruction.  Measured,
@@ -403,14 +412,9 @@ template <typename R> static int launch_typed(pond_ctx* c, const void* const* in
     case POND_D3Q27:
       if constexpr (std::is_same<R, float>::value) {
         if (c->p.interp >= POND_LAGR2 && c->p.interp <= POND_LAGR4) {
-          dim3 blk(d27::TX, d27::TY, d27::TZ);
-          dim3 grd((a.nx + d27::TX - 1) / d27::TX, (a.ny + d27::TY - 1) / d27::TY, (a.nz + d27::TZ - 1) / d27::TZ);
-          void (*kern)(StepArgs<float>) = c->p.interp == POND_LAGR2   ? d27::pull_d3q27_tile_kernel<2>
-                                          : c->p.interp == POND_LAGR3 ? d27::pull_d3q27_tile_kernel<3>
-                                                                      : d27::pull_d3q27_tile_kernel<4>;
-          e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d27::SMEM_BYTES);
-          if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute");
-          e = launch_early(kern, grd, blk, d27::SMEM_BYTES, s, a);
+          e = c->p.interp == POND_LAGR2   ? launch_d3q27_tile<2>(a, s)
+              : c->p.interp == POND_LAGR3 ? launch_d3q27_tile<3>(a, s)
+                                          : launch_d3q27_tile<4>(a, s);
           if (e != cudaSuccess) return cuda_fail(e, "step kernel launch");
           break;
         }

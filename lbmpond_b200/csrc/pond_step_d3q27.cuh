@@ -4,7 +4,8 @@
 // Same arithmetic as pull_point_kernel (steps.cu:356-588 LBMpull with
 // propagate<N>, N = 2, 3, 4), organised for the SM:
 //
-//  * a CTA owns an 8 x 4 x 4 tile of nodes and stages the tile plus a halo of
+//  * a CTA owns an 8 x 4 x 4 tile of nodes (order 3: 32 x 4 x 2, see Tile) and
+//    stages the tile plus a halo of
 //    2 nodes per side (12 x 8 x 8 nodes) once per step, node-major: a staged
 //    node's 27 populations are contiguous and 16-byte aligned (a 28-float
 //    stride, 86 KB), so a lane fetches a stencil node with seven 16-byte
@@ -35,10 +36,11 @@
 //    every offset (a class a lane does not weight there has weight 0), except
 //    at the two ends of the usual z window (contract_tile);
 //  * once only a few lanes of a warp still iterate, the warp serves their nodes
-//    one at a time, a stencil column per lane: a node that runs to the
-//    iteration cap then takes 2 us per iteration instead of 11 to 20, which is
-//    what the end of a step waited for (two nodes of a 128^3 vortex at the cap:
-//    3.87 -> 3.38 ms; two steps with energy populations at 64^3: 4.39 -> 2.46 ms);
+//    one at a time, a stencil column per lane, with the same roundings: a node
+//    that runs to the iteration cap then takes 2 us per iteration instead of 11
+//    to 20, which is what the end of a step waited for (128^3 vortex with nodes
+//    at the cap, order 3: 4.22 -> 3.88 ms; two steps with energy populations at
+//    64^3: 4.11 -> 2.58 ms);
 //  * the z and y contractions run as two-wide float32 multiply-adds on pairs
 //    of populations that the staged layout keeps in neighbouring registers
 //    (slot27): 45 instructions per stencil node instead of 81, for the same
@@ -62,19 +64,49 @@
 namespace pond {
 namespace d27 {
 
-constexpr int TX = 8, TY = 4, TZ = 4, H = 2;
-constexpr int SX = TX + 2 * H, SY = TY + 2 * H, SZ = TZ + 2 * H;
-constexpr int SN = SX * SY * SZ;  // 768 staged nodes
-constexpr int NS = 28;            // floats per staged node: its 27 R-gauge populations and a pad
-constexpr int THREADS = TX * TY * TZ;
-// staged nodes node-major (a node's populations contiguous, 16-byte aligned:
-// seven 16-byte loads per stencil node; the 28-word stride keeps the eight
-// lanes of each 16-byte load phase on distinct banks), then the iterate's
-// populations of every lane
-constexpr size_t SMEM_BYTES =
-    size_t(NS) * SN * sizeof(float) + size_t(27) * THREADS * sizeof(float) + size_t(THREADS / 32) * 28 * sizeof(float) +
-    size_t(3) * SN * sizeof(float);
-static_assert(2 * (SMEM_BYTES + 2048) <= 233472, "two CTAs must fit in the 228 KB of an SM");
+constexpr int H = 2;    // halo
+constexpr int NS = 28;  // floats per staged node: its 27 R-gauge populations and a pad
+// Scratch of a warp for contract_node_by_warp that takes `rows` rows of five
+// stencil columns at a time, in floats (27 each, from 16-byte boundaries).
+__host__ __device__ constexpr int served_floats(int rows) { return (5 * 27 * rows + 3) / 4 * 4; }
+
+// The tile of order N and its shared memory: the staged nodes (node-major, a
+// node's populations contiguous, 16-byte aligned: seven 16-byte loads per
+// stencil node; the 28-word stride keeps the eight lanes of each 16-byte load
+// phase on distinct banks), the iterate's populations of every lane, the
+// warps' scratch and the staged velocities.
+//
+// Orders 2 and 4: 8 x 4 x 4, two CTAs per SM.  Order 3: 32 x 4 x 2, one CTA of
+// eight warps, its velocities staged in the iterates' place.  A quadratic
+// window is chosen by rounding (x) and jumps where two windows meet, so a node
+// whose iterates cycle between two of them turns the last digit of a transfer
+// into 1e-3 of its populations; the reference gauge decides those digits, and
+// order 3 keeps the gauge of 32 x 4 x 2 blocks that its results were checked
+// with (26 boxes of 26 to 110 nodes a side, 1 to 8 steps: with an 8 x 4 x 4
+// tile's gauge two came out 1e-6 and 2.9e-6 off float64 instead of 3e-7, and
+// two others 2e-7 instead of 1.5e-6).  The wider tile costs a 128^3 vortex 3.88
+// instead of 3.33 ms per step.
+template <int N> struct Tile {
+  static constexpr int TX = N == 3 ? 32 : 8, TY = 4, TZ = N == 3 ? 2 : 4;
+  static constexpr int SX = TX + 2 * H, SY = TY + 2 * H, SZ = TZ + 2 * H;
+  static constexpr int SN = SX * SY * SZ;  // staged nodes
+  static constexpr int THREADS = TX * TY * TZ, WARPS = THREADS / 32, CTAS = N == 3 ? 1 : 2;
+  static constexpr bool kOwnLater = N == 3;
+  // the warps' scratch takes the velocities' place, or what is left of the SM's shared memory
+  static constexpr int ROWS = N == 3 ? 2 : 5, SERVED = served_floats(ROWS);
+  static constexpr int OFF_OWN = NS * SN, OFF_S = OFF_OWN + 27 * THREADS, OFF_U = kOwnLater ? OFF_OWN : OFF_S;
+  static constexpr size_t SMEM_BYTES =
+      size_t(kOwnLater || 3 * SN < SERVED * WARPS ? OFF_S + SERVED * WARPS : OFF_S + 3 * SN) * sizeof(float);
+  static_assert(!kOwnLater || 3 * SN <= 27 * THREADS, "the velocities must fit the iterates' place");
+  static_assert(CTAS * (SMEM_BYTES + 1024 + 2432) <= 233472, "the CTAs must fit in the 228 KB of an SM");
+  // nodes: a warp takes an 8 x 4 patch of a z plane
+  static __device__ __forceinline__ int lx(int tid) { return (tid & 7) + 8 * ((tid >> 5) % (TX / 8)); }
+  static __device__ __forceinline__ int ly(int tid) { return (tid >> 3) & 3; }
+  static __device__ __forceinline__ int lz(int tid) { return (tid >> 5) / (TX / 8); }
+  static __device__ __forceinline__ int thread_of(int x, int y, int z) {
+    return (x & 7) + 8 * y + 32 * ((x >> 3) + (TX / 8) * z);
+  }
+};
 
 // Slot of class (k1, k2, k3) in a staged node: the contractions along z and y
 // run on pairs of populations (two-wide float32 multiply-adds), so the
@@ -141,11 +173,14 @@ template <typename R> __device__ __forceinline__ void node_to_ref(R v[27], const
   }
 }
 
-// node_to_ref of a staged node in its slots, non-finite populations counted
-// as 0 (all of them when !ok): pairs of classes k1 = +, - through the z and y
-// passes and pairs of target classes i1 = +, - in the x pass, 153
-// instructions for the 243 multiply-adds.  `raw` (null, or the node's column
-// of the iterates, `stride` floats apart) gets the populations as they were.
+// node_to_ref of a staged node in its slots, with the same roundings (the
+// axes in the same order; a node beyond the halo goes through node_to_ref, and
+// nodes whose iterates cycle between two windows turn a last digit into 1e-3):
+// non-finite populations count as 0 (all of them when !ok).  Pairs of target
+// classes i1 = +, - from the x pass on, pairs i2 = +, - of i1 = 0 from the y
+// pass on: 144 instructions for the 243 multiply-adds.  `raw` (null, or the
+// node's column of the iterates, `stride` floats apart) gets the populations
+// as they were.
 __device__ __forceinline__ void staged_to_ref(float* node, bool ok, const float s[3], const float r[3], float* raw,
                                               int stride) {
   float e[28];
@@ -161,45 +196,53 @@ __device__ __forceinline__ void staged_to_ref(float* node, bool ok, const float 
 #pragma unroll
   for (int q = 0; q < 27; q++) e[q] = (ok && fabsf(e[q]) <= 3.402823466e38f) ? e[q] : 0.f;
   float B[3][3];
-  float2 P[3][3], Q[3];  // [k2][i3] of k1 = +, -; [i3] of k1 = 0, k2 = +, -
-  float S[3];            // [i3] of k1 = k2 = 0
-  basis_rows(s[2], r[2], B);
+  float2 P[3][3];  // [k2][k3] of i1 = +, -
+  float Z[3][3];   // [k2][k3] of i1 = 0
+  basis_rows(s[0], r[0], B);
+  {
+    const float2 c0 = make_float2(B[1][0], B[2][0]), c1 = make_float2(B[1][1], B[2][1]), c2 = make_float2(B[1][2], B[2][2]);
 #pragma unroll
-  for (int i = 0; i < 3; i++) {
-    const auto row = [&](int slot, int step) {  // sum_k3 B[i][k3] of the pairs at slot, slot + step, ..
-      float2 o = __fmul2_rn(make_float2(B[i][0], B[i][0]), make_float2(e[slot], e[slot + 1]));
-      o = __ffma2_rn(make_float2(B[i][1], B[i][1]), make_float2(e[slot + step], e[slot + step + 1]), o);
-      return __ffma2_rn(make_float2(B[i][2], B[i][2]), make_float2(e[slot + 2 * step], e[slot + 2 * step + 1]), o);
-    };
+    for (int k2 = 0; k2 < 3; k2++)
 #pragma unroll
-    for (int k2 = 0; k2 < 3; k2++) P[k2][i] = row(slot27(1, k2, 0), slot27(1, 0, 1) - slot27(1, 0, 0));
-    Q[i] = row(slot27(0, 1, 0), slot27(0, 1, 1) - slot27(0, 1, 0));
-    S[i] = fmaf(B[i][2], e[26], fmaf(B[i][1], e[25], B[i][0] * e[24]));
+      for (int k3 = 0; k3 < 3; k3++) {
+        const float z = e[slot27(0, k2, k3)], p = e[slot27(1, k2, k3)], m = e[slot27(2, k2, k3)];
+        Z[k2][k3] = fmaf(B[0][2], m, fmaf(B[0][1], p, B[0][0] * z));
+        P[k2][k3] = __ffma2_rn(c2, make_float2(m, m), __ffma2_rn(c1, make_float2(p, p), __fmul2_rn(c0, make_float2(z, z))));
+      }
   }
   basis_rows(s[1], r[1], B);
-  float2 P2[3][3];  // [i2][i3] of k1 = +, -
-  float Z[3][3];    // [i2][i3] of k1 = 0
+  float2 P2[3][3], Q[3];  // [i2][k3] of i1 = +, -; [k3] of i1 = 0, i2 = +, -
+  float S[3];             // [k3] of i1 = i2 = 0
+  {
+    const float2 c0 = make_float2(B[1][0], B[2][0]), c1 = make_float2(B[1][1], B[2][1]), c2 = make_float2(B[1][2], B[2][2]);
 #pragma unroll
-  for (int i2 = 0; i2 < 3; i2++)
+    for (int k3 = 0; k3 < 3; k3++) {
 #pragma unroll
-    for (int i3 = 0; i3 < 3; i3++) {
-      const float b0 = B[i2][0], b1 = B[i2][1], b2 = B[i2][2];
-      P2[i2][i3] = __ffma2_rn(make_float2(b2, b2), P[2][i3],
-                              __ffma2_rn(make_float2(b1, b1), P[1][i3], __fmul2_rn(make_float2(b0, b0), P[0][i3])));
-      Z[i2][i3] = fmaf(b2, Q[i3].y, fmaf(b1, Q[i3].x, b0 * S[i3]));
+      for (int i2 = 0; i2 < 3; i2++) {
+        const float b0 = B[i2][0], b1 = B[i2][1], b2 = B[i2][2];
+        P2[i2][k3] = __ffma2_rn(make_float2(b2, b2), P[2][k3],
+                                __ffma2_rn(make_float2(b1, b1), P[1][k3], __fmul2_rn(make_float2(b0, b0), P[0][k3])));
+      }
+      const float z = Z[0][k3], p = Z[1][k3], m = Z[2][k3];
+      S[k3] = fmaf(B[0][2], m, fmaf(B[0][1], p, B[0][0] * z));
+      Q[k3] = __ffma2_rn(c2, make_float2(m, m), __ffma2_rn(c1, make_float2(p, p), __fmul2_rn(c0, make_float2(z, z))));
     }
-  basis_rows(s[0], r[0], B);
-  const float2 c0 = make_float2(B[1][0], B[2][0]), c1 = make_float2(B[1][1], B[2][1]), c2 = make_float2(B[1][2], B[2][2]);
+  }
+  basis_rows(s[2], r[2], B);
 #pragma unroll
-  for (int i2 = 0; i2 < 3; i2++)
+  for (int i3 = 0; i3 < 3; i3++) {
+    const float b0 = B[i3][0], b1 = B[i3][1], b2 = B[i3][2];
+    const auto pair = [&](const float2 v[3], int slot) {
+      const float2 o = __ffma2_rn(make_float2(b2, b2), v[2],
+                                  __ffma2_rn(make_float2(b1, b1), v[1], __fmul2_rn(make_float2(b0, b0), v[0])));
+      e[slot] = o.x;
+      e[slot + 1] = o.y;
+    };
 #pragma unroll
-    for (int i3 = 0; i3 < 3; i3++) {
-      const float z = Z[i2][i3], p = P2[i2][i3].x, m = P2[i2][i3].y;
-      e[slot27(0, i2, i3)] = fmaf(B[0][2], m, fmaf(B[0][1], p, B[0][0] * z));
-      const float2 o = __ffma2_rn(c2, make_float2(m, m), __ffma2_rn(c1, make_float2(p, p), __fmul2_rn(c0, make_float2(z, z))));
-      e[slot27(1, i2, i3)] = o.x;
-      e[slot27(2, i2, i3)] = o.y;
-    }
+    for (int i2 = 0; i2 < 3; i2++) pair(P2[i2], slot27(1, i2, i3));
+    pair(Q, slot27(0, 1, i3));
+    e[slot27(0, 0, i3)] = fmaf(b2, S[2], fmaf(b1, S[1], b0 * S[0]));
+  }
   e[27] = 0.f;
 #pragma unroll
   for (int q = 0; q < 7; q++) s4[q] = make_float4(e[4 * q], e[4 * q + 1], e[4 * q + 2], e[4 * q + 3]);
@@ -229,41 +272,59 @@ __device__ __forceinline__ void copy_node(const float* f, long long N, long long
   }
 }
 
-// moments_and_test for the float32 tiles: the node's previous populations in
-// shared memory (`f0`, `stride` floats apart, replaced by acc), the sums of
-// each class of each axis first (93 float64 operations instead of 190), and
-// the difference of the populations in float32, where it is exact whenever the
-// test is close.
+// moments_and_test for the float32 tiles: the node's previous populations lie
+// in shared memory (`f0`, `stride` floats apart, replaced by acc), and the
+// difference of the populations is taken in float32.
+// Order 3 forms its sums in moments_and_test's order, so that its results stay
+// those of the node-by-node sums to the last bit (128^3: 1 % of the step).
+template <int N>
 __device__ __forceinline__ bool tile_moments_and_test(const StepArgs<float>& a, const float acc[27], float* f0, int stride,
                                                       double C, double& rho0, double U[3], double& T) {
   using L = Lattice<POND_D3Q27>;
-  double sx[3] = {0, 0, 0}, sy[3] = {0, 0, 0}, sz[3] = {0, 0, 0};
   bool ok = true;
 #pragma unroll
-  for (int cx = 0; cx < 3; cx++)
+  for (int t = 0; t < 27; t++) {
+    const double nv = acc[t];
+    ok = ok && !(double(fabsf(acc[t] - f0[t * stride])) >= a.tol_abs + a.tol_rel * fabs(nv));
+  }
+  double m[4] = {0, 0, 0, 0}, rho = 0;
+  if constexpr (N == 3) {
 #pragma unroll
-    for (int cy = 0; cy < 3; cy++) {
-      double row = 0;
-#pragma unroll
-      for (int cz = 0; cz < 3; cz++) {
-        const int t = (cx * 3 + cy) * 3 + cz;
-        const double nv = acc[t];
-        row += nv;
-        sz[cz] += nv;
-        ok = ok && !(double(fabsf(acc[t] - f0[t * stride])) >= a.tol_abs + a.tol_rel * fabs(nv));
-        f0[t * stride] = acc[t];
-      }
-      sx[cx] += row;
-      sy[cy] += row;
+    for (int t = 0; t < 27; t++) {
+      const double fv = acc[t];
+      const double vx = C * L::xi1(t / 9) + U[0], vy = C * L::xi1(t / 3 % 3) + U[1], vz = C * L::xi1(t % 3) + U[2];
+      rho += fv;
+      m[0] += fv * vx; m[1] += fv * vy; m[2] += fv * vz;
+      m[3] += fv * (vx * vx + vy * vy + vz * vz);
+      f0[t * stride] = acc[t];
     }
-  const double rho = sx[0] + sx[1] + sx[2];
-  double m[4] = {0, 0, 0, 0};
+  } else {
+    // the sums of each class of each axis first: 93 operations instead of 190
+    double sx[3] = {0, 0, 0}, sy[3] = {0, 0, 0}, sz[3] = {0, 0, 0};
 #pragma unroll
-  for (int c = 0; c < 3; c++) {
-    const double vx = C * L::xi1(c) + U[0], vy = C * L::xi1(c) + U[1], vz = C * L::xi1(c) + U[2];
-    const double px = sx[c] * vx, py = sy[c] * vy, pz = sz[c] * vz;
-    m[0] += px; m[1] += py; m[2] += pz;
-    m[3] += px * vx + py * vy + pz * vz;
+    for (int cx = 0; cx < 3; cx++)
+#pragma unroll
+      for (int cy = 0; cy < 3; cy++) {
+        double row = 0;
+#pragma unroll
+        for (int cz = 0; cz < 3; cz++) {
+          const int t = (cx * 3 + cy) * 3 + cz;
+          const double nv = acc[t];
+          row += nv;
+          sz[cz] += nv;
+          f0[t * stride] = acc[t];
+        }
+        sx[cx] += row;
+        sy[cy] += row;
+      }
+    rho = sx[0] + sx[1] + sx[2];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const double vx = C * L::xi1(c) + U[0], vy = C * L::xi1(c) + U[1], vz = C * L::xi1(c) + U[2];
+      const double px = sx[c] * vx, py = sy[c] * vy, pz = sz[c] * vz;
+      m[0] += px; m[1] += py; m[2] += pz;
+      m[3] += px * vx + py * vy + pz * vz;
+    }
   }
   if (rho != 0) {
     const double ir = 1.0 / rho;
@@ -467,18 +528,32 @@ __device__ __forceinline__ void contract_tile(const float* centre, int sx, int s
   }
 }
 
-// The same iterate for one node by the whole warp: lane 5 (oy + 2) + ox + 2
-// contracts the stencil column at (ox, oy) through all three axes, and the
-// lanes' sums are reduced so that lane t < 27 returns population t.  All
-// arguments are the node's (warp-uniform).  Used when few lanes of a warp
-// still iterate: the warp's contraction of all its lanes costs the same
-// however few they are (about 11,000 instructions at N = 4, 1,200 here per node).
-template <int N>
-__device__ __forceinline__ float contract_node_by_warp(const float* centre, int sx, int sxy, const int lo[3],
-                                                       const int hi[3], const int ro[3][3], const float wt[3][3][N],
-                                                       const float bq[3], float ainv, int lane) {
+// What contract_node_by_warp needs of its node, in the warp's scratch.
+template <int N> struct alignas(16) ServedNode {
+  float wt[3][3][N], bq[3], ainv;
+  int ro[3][3], lo[3], hi[3], centre;
+};
+static_assert(sizeof(ServedNode<4>) <= served_floats(1) * sizeof(float), "the scratch holds a node's windows");
+
+// The same iterate for one node by the whole warp, with contract_tile's
+// roundings: lane 5 (oy + 2) + ox + 2 sums the stencil column at (ox, oy) along
+// z; then, ROWS rows of columns at a time, the sums go through shared memory to
+// lane 9 k1 + 3 i2 + i3, which takes them along y, and to lane 9 i1 + 3 i2 + i3
+// by shuffle along x.  Every sum runs over the same terms in the same order as in
+// contract_tile (whose further offsets have weight 0), so a node's result does
+// not depend on how many of its neighbours still iterate.  The node comes in
+// `scratch` and its populations go there.  Used when few lanes of a warp still
+// iterate: the warp's contraction of all its lanes costs the same however few
+// they are (about 11,000 instructions at N = 4).  Not inlined: the registers it
+// needs would be taken from the contraction of full warps (256^3: 28.5 ms, 31.6
+// inlined).  Five rows at a time instead of one: 28.5 -> 28.3 ms there, two steps
+// with energy populations at 64^3 2.73 -> 2.65 (three rows).
+template <int N, int ROWS>
+__device__ __noinline__ void contract_node_by_warp(const float* staged, int sx, int sxy, float* scratch) {
+  const int lane = threadIdx.x & 31;
+  const ServedNode<N>& node = *reinterpret_cast<const ServedNode<N>*>(scratch);
   const int ox = lane < 25 ? lane % 5 - 2 : 0, oy = lane < 25 ? lane / 5 - 2 : 0;
-  const bool part = lane < 25 && ox >= lo[0] && ox <= hi[0] && oy >= lo[1] && oy <= hi[1];
+  const int xlo = max(node.lo[0], -H), xhi = min(node.hi[0], H), ylo = node.lo[1], yhi = node.hi[1];
   float2 Zp[3][3], Zq[3];
   float Zs[3], G[3][3];
 #pragma unroll
@@ -488,84 +563,117 @@ __device__ __forceinline__ float contract_node_by_warp(const float* centre, int 
     Zq[i] = make_float2(0.f, 0.f);
     Zs[i] = 0.f;
   }
-  basis_rows(bq[2], ainv, G);
+  const float ainv = node.ainv;
+  basis_rows(node.bq[2], ainv, G);
+  {
+    const float* col = staged + (node.centre + oy * sx + ox) * NS;
+    const int zlo = node.lo[2], zhi = node.hi[2];
 #pragma unroll
-  for (int oz = -H; oz <= H; oz++) {
-    if (oz < lo[2] || oz > hi[2]) continue;
-    float w[3];
+    for (int oz = -H; oz <= H; oz++) {
+      if (oz < zlo || oz > zhi) continue;
+      float w[3];
 #pragma unroll
-    for (int c = 0; c < 3; c++) w[c] = wpick<N>(wt[2][c], ro[2][c], oz);
-    column_node<true, true>(centre + (oz * sxy + oy * sx + ox) * NS, G, w, Zp, Zq, Zs);
-  }
-  float Y[3][9];  // [k1][3 i2 + i3]
-  basis_rows(bq[1], ainv, G);
-#pragma unroll
-  for (int i2 = 0; i2 < 3; i2++) {
-    const float w = wpick<N>(wt[1][i2], ro[1][i2], oy);
-    const float g0 = w * G[i2][0], g1 = w * G[i2][1], g2 = w * G[i2][2];
-#pragma unroll
-    for (int i3 = 0; i3 < 3; i3++) {
-      Y[0][3 * i2 + i3] = fmaf(g2, Zq[i3].y, fmaf(g1, Zq[i3].x, g0 * Zs[i3]));
-      Y[1][3 * i2 + i3] = fmaf(g2, Zp[i3][2].x, fmaf(g1, Zp[i3][1].x, g0 * Zp[i3][0].x));
-      Y[2][3 * i2 + i3] = fmaf(g2, Zp[i3][2].y, fmaf(g1, Zp[i3][1].y, g0 * Zp[i3][0].y));
+      for (int c = 0; c < 3; c++) w[c] = wpick<N>(node.wt[2][c], node.ro[2][c], oz);
+      column_node<true, true>(col + oz * sxy * NS, G, w, Zp, Zq, Zs);
     }
   }
-  float v[32];
-  basis_rows(bq[0], ainv, G);
+  // this lane's classes along y and x: the rows i2 and i1 of the bases, the windows and their weights
+  const int i1 = min(lane / 9, 2), i2 = (lane / 3) % 3, i3 = lane % 3;
+  float Gy[3], Gx[3], wy[N], wx[N];
+  const auto row = [](float B[3][3], int i, float out[3]) {
 #pragma unroll
-  for (int i1 = 0; i1 < 3; i1++) {
-    const float w = wpick<N>(wt[0][i1], ro[0][i1], ox);
+    for (int k = 0; k < 3; k++) out[k] = i == 0 ? B[0][k] : i == 1 ? B[1][k] : B[2][k];
+  };
+  basis_rows(node.bq[1], ainv, G);
+  row(G, i2, Gy);
+  basis_rows(node.bq[0], ainv, G);
+  row(G, i1, Gx);
 #pragma unroll
-    for (int i23 = 0; i23 < 9; i23++) {
-      const float t = w * fmaf(G[i1][2], Y[2][i23], fmaf(G[i1][1], Y[1][i23], G[i1][0] * Y[0][i23]));
-      v[9 * i1 + i23] = part ? t : 0.f;
-    }
+  for (int k = 0; k < N; k++) {
+    wy[k] = node.wt[1][i2][k];
+    wx[k] = node.wt[0][i1][k];
   }
+  const int roy = node.ro[1][i2], rox = node.ro[0][i1];
+  __syncwarp();  // the node has been read
+  // column slots: pairs [2 (3 i3 + k2) + k1 - 1] of k1 = +, -, then those of k1 = 0 as [18 + 3 i3 + k2]
+  const int from = i1 > 0 ? 6 * i3 + i1 - 1 : 18 + 3 * i3, step = i1 > 0 ? 2 : 1;  // k1 = i1 here
+  float out = 0.f;
+#pragma unroll 1
+  for (int p0 = xlo; p0 <= xhi; p0 += ROWS) {
+    if (lane < 25 && ox >= p0 && ox < p0 + ROWS) {
+      float* col = scratch + (5 * (ox - p0) + oy + H) * 27;
 #pragma unroll
-  for (int t = 27; t < 32; t++) v[t] = 0.f;
-  // halve the values and the lanes they are summed over: lane t ends with the sum of v[t]
+      for (int i = 0; i < 3; i++) {
 #pragma unroll
-  for (int h = 16; h > 0; h >>= 1)
-#pragma unroll
-    for (int t = 0; t < h; t++) {
-      const bool up = lane & h;
-      const float give = up ? v[t] : v[t + h], keep = up ? v[t + h] : v[t];
-      v[t] = keep + __shfl_xor_sync(0xffffffffu, give, h);
+        for (int k2 = 0; k2 < 3; k2++) {
+          col[2 * (3 * i + k2)] = Zp[i][k2].x;
+          col[2 * (3 * i + k2) + 1] = Zp[i][k2].y;
+        }
+        col[18 + 3 * i] = Zs[i];
+        col[18 + 3 * i + 1] = Zq[i].x;
+        col[18 + 3 * i + 2] = Zq[i].y;
+      }
     }
-  return v[0];
+    __syncwarp();
+    float Y[ROWS];
+#pragma unroll
+    for (int r = 0; r < ROWS; r++) Y[r] = 0.f;
+#pragma unroll
+    for (int py = -H; py <= H; py++) {
+      if (py < ylo || py > yhi) continue;  // warp-uniform
+      const float* col = scratch + (py + H) * 27 + from;
+      const float w = wpick<N>(wy, roy, py);
+      const float g0 = w * Gy[0], g1 = w * Gy[1], g2 = w * Gy[2];
+#pragma unroll
+      for (int r = 0; r < ROWS; r++)  // rows past the last are not used
+        Y[r] = fmaf(g2, col[135 * r + 2 * step], fmaf(g1, col[135 * r + step], fmaf(g0, col[135 * r], Y[r])));
+    }
+    const int at = 3 * i2 + i3;
+#pragma unroll
+    for (int r = 0; r < ROWS; r++) {
+      if (p0 + r > xhi) break;
+      const float w = wpick<N>(wx, rox, p0 + r);
+      const float g0 = w * Gx[0], g1 = w * Gx[1], g2 = w * Gx[2];
+      const float y0 = __shfl_sync(0xffffffffu, Y[r], at), y1 = __shfl_sync(0xffffffffu, Y[r], 9 + at),
+                  y2 = __shfl_sync(0xffffffffu, Y[r], 18 + at);
+      out = fmaf(g2, y2, fmaf(g1, y1, fmaf(g0, y0, out)));
+    }
+    __syncwarp();
+  }
+  if (lane < 27) scratch[lane] = out;
+  __syncwarp();
 }
 
 // The lanes of `live`, one after another, through contract_node_by_warp; each
 // gets its node's populations in acc.  `centre`: the lane's staged node;
-// `scratch`: 27 floats of the warp.
-template <int N>
+// `scratch`: served_floats(ROWS) floats of the warp, 16-byte aligned.
+template <int N, int ROWS>
 __device__ __forceinline__ void contract_live_lanes(unsigned live, const float* staged, int centre, int sx, int sxy,
                                                     const int lo[3], const int hi[3], const int ro[3][3],
                                                     const float wt[3][3][N], const float bq[3], float ainv,
                                                     float* scratch, float acc[27]) {
-  const int lane = (threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z)) & 31;
+  const int lane = threadIdx.x & 31;
 #pragma unroll 1
   for (; live; live &= live - 1) {
     const int src = __ffs(live) - 1;
-    int lo_s[3], hi_s[3], ro_s[3][3];
-    float wt_s[3][3][N], bq_s[3];
+    if (lane == src) {
+      ServedNode<N> node;
 #pragma unroll
-    for (int ax = 0; ax < 3; ax++) {
-      lo_s[ax] = __shfl_sync(0xffffffffu, lo[ax], src);
-      hi_s[ax] = __shfl_sync(0xffffffffu, hi[ax], src);
-      bq_s[ax] = __shfl_sync(0xffffffffu, bq[ax], src);
+      for (int ax = 0; ax < 3; ax++) {
+        node.lo[ax] = lo[ax]; node.hi[ax] = hi[ax]; node.bq[ax] = bq[ax];
 #pragma unroll
-      for (int c = 0; c < 3; c++) {
-        ro_s[ax][c] = __shfl_sync(0xffffffffu, ro[ax][c], src);
+        for (int c = 0; c < 3; c++) {
+          node.ro[ax][c] = ro[ax][c];
 #pragma unroll
-        for (int k = 0; k < N; k++) wt_s[ax][c][k] = __shfl_sync(0xffffffffu, wt[ax][c][k], src);
+          for (int k = 0; k < N; k++) node.wt[ax][c][k] = wt[ax][c][k];
+        }
       }
+      node.ainv = ainv;
+      node.centre = centre;
+      *reinterpret_cast<ServedNode<N>*>(scratch) = node;
     }
-    const float a_s = __shfl_sync(0xffffffffu, ainv, src);
-    const float* c_s = staged + __shfl_sync(0xffffffffu, centre, src) * NS;
-    const float r = contract_node_by_warp<N>(c_s, sx, sxy, lo_s, hi_s, ro_s, wt_s, bq_s, a_s, lane);
-    if (lane < 27) scratch[lane] = r;
     __syncwarp();
+    contract_node_by_warp<N, ROWS>(staged, sx, sxy, scratch);
     if (lane == src)
 #pragma unroll
       for (int t = 0; t < 27; t++) acc[t] = scratch[t];
@@ -575,8 +683,9 @@ __device__ __forceinline__ void contract_live_lanes(unsigned live, const float* 
 
 // Live lanes at which the warp serves nodes one by one: the serial iteration
 // costs about 11,000 / 6,500 / 3,000 instructions (N = 4 / 3 / 2), a node by
-// the warp 1,200.  8 / 5 / 2 lanes measured 0.4-1.5 % faster than 5 / 3 / 1.
-template <int N> __host__ __device__ constexpr int few_lanes() { return N == 4 ? 8 : N == 3 ? 5 : 2; }
+// the warp 1,300 and its exchanges.  4 to 6 lanes (N = 4) and 3 or 4 (N = 3)
+// are within 0.7 % of each other from 32^3 to 256^3, 8 lanes 0.5-4 % slower.
+template <int N> __host__ __device__ constexpr int few_lanes() { return N == 4 ? 5 : N == 3 ? 3 : 2; }
 
 // Partial record of the step sums, updated instead of the context's sums
 // when the kernel runs without a context (kPartials = true; a.sums then
@@ -590,11 +699,11 @@ struct BlockPartial {
   int pad;
 };
 
-__device__ __forceinline__ void add_block_partial(NodeSums s, BlockPartial* out) {
-  __shared__ double pd[6][THREADS / 32];
-  __shared__ unsigned long long pu[3][THREADS / 32];
-  __shared__ int pm[THREADS / 32];
-  const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
+template <int WARPS> __device__ __forceinline__ void add_block_partial(NodeSums s, BlockPartial* out) {
+  __shared__ double pd[6][WARPS];
+  __shared__ unsigned long long pu[3][WARPS];
+  __shared__ int pm[WARPS];
+  const int tid = threadIdx.x;
   const int warp = tid >> 5;
   double v[6] = {s.mass, s.m0, s.m1, s.m2, s.enrg, s.k};
 #pragma unroll
@@ -613,7 +722,7 @@ __device__ __forceinline__ void add_block_partial(NodeSums s, BlockPartial* out)
   __syncthreads();
   if (tid == 0) {
     BlockPartial b = {};
-    for (int w = 0; w < THREADS / 32; w++) {
+    for (int w = 0; w < WARPS; w++) {
       b.mass += pd[0][w]; b.mom[0] += pd[1][w]; b.mom[1] += pd[2][w]; b.mom[2] += pd[3][w];
       b.enrg += pd[4][w]; b.k += pd[5][w];
       b.niter_sum += pu[0][w]; b.nonconv += pu[1][w]; b.work += pu[2][w];
@@ -633,12 +742,15 @@ __device__ __forceinline__ void add_block_partial(NodeSums s, BlockPartial* out)
 }
 
 template <int N, bool kPartials = false>
-__global__ void __launch_bounds__(THREADS, 2) pull_d3q27_tile_kernel(StepArgs<float> a) {
+__global__ void __launch_bounds__(Tile<N>::THREADS, Tile<N>::CTAS) pull_d3q27_tile_kernel(StepArgs<float> a) {
   using L = Lattice<POND_D3Q27>;
+  using Ti = Tile<N>;
+  constexpr int SX = Ti::SX, SY = Ti::SY, SN = Ti::SN, THREADS = Ti::THREADS;
   extern __shared__ __align__(16) float sm[];
-  const int tid = threadIdx.x + TX * (threadIdx.y + TY * threadIdx.z);
-  const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY, z0 = blockIdx.z * TZ;
-  float* su = sm + NS * SN + 27 * THREADS + (THREADS / 32) * 28;
+  const int tid = threadIdx.x;
+  float* own = sm + Ti::OFF_OWN;
+  float* su = sm + Ti::OFF_U;
+  const int x0 = blockIdx.x * Ti::TX, y0 = blockIdx.y * Ti::TY, z0 = blockIdx.z * Ti::TZ;
   // launched while the step before still runs (launch_early): let the next one
   // come, then wait for the step before to be complete and visible
   cudaTriggerProgrammaticLaunchCompletion();
@@ -668,9 +780,9 @@ __global__ void __launch_bounds__(THREADS, 2) pull_d3q27_tile_kernel(StepArgs<fl
   float uref[3], icref;
   {
     bool rv[3];
-    const int gx = resolve_axis(x0 + TX / 2, a.nx, a.bc[0], rv[0]);
-    const int gy = resolve_axis(y0 + TY / 2, a.ny, a.bc[1], rv[1]);
-    const int gz = resolve_axis(z0 + TZ / 2, a.nz, a.bc[2], rv[2]);
+    const int gx = resolve_axis(x0 + Ti::TX / 2, a.nx, a.bc[0], rv[0]);
+    const int gy = resolve_axis(y0 + Ti::TY / 2, a.ny, a.bc[1], rv[1]);
+    const int gz = resolve_axis(z0 + Ti::TZ / 2, a.nz, a.bc[2], rv[2]);
     const long long g = gx + (long long)a.nx * (gy + (long long)a.ny * gz);
     const float T = a.g_in[3 * a.N + g];
     const float cc = copysignf(sqrtf(fabsf(T) * (float)(1.0 / L::TLat)), T);
@@ -710,20 +822,27 @@ __global__ void __launch_bounds__(THREADS, 2) pull_d3q27_tile_kernel(StepArgs<fl
                          ok ? (u[2] - uref[2]) * icref : 0.f};
     const float rq[3] = {r, r, r};
     // a node of the tile leaves its populations where its thread keeps its iterate
-    const int tx = hx - H, ty = hy - H, tz = hz - H;
-    const bool own = tx >= 0 && tx < TX && ty >= 0 && ty < TY && tz >= 0 && tz < TZ;
-    staged_to_ref(sm + i * NS, ok, sq, rq, own ? sm + NS * SN + tx + TX * (ty + TY * tz) : nullptr, THREADS);
+    float* raw = nullptr;
+    if constexpr (!Ti::kOwnLater) {
+      const int tx = hx - H, ty = hy - H, tz = hz - H;
+      if (tx >= 0 && tx < Ti::TX && ty >= 0 && ty < Ti::TY && tz >= 0 && tz < Ti::TZ) raw = own + Ti::thread_of(tx, ty, tz);
+    }
+    staged_to_ref(sm + i * NS, ok, sq, rq, raw, THREADS);
   }
   __syncthreads();
 
-  const int lx = threadIdx.x, ly = threadIdx.y, lz = threadIdx.z;
+  const int lx = Ti::lx(tid), ly = Ti::ly(tid), lz = Ti::lz(tid);
   const int x = x0 + lx, y = y0 + ly, z = z0 + lz;
   const bool active = x < a.nx && y < a.ny && z < a.nz;
   NodeSums ns = {0, 0, 0, 0, 0, 0, 0ull, 0ull, 0ull, 0};
   const long long idx = active ? x + (long long)a.nx * (y + (long long)a.ny * z) : 0;
   // the node's current populations live in shared memory between iterations,
   // which keeps them out of the loop's registers
-  float* f0s = sm + NS * SN + tid;
+  float* f0s = own + tid;
+  if constexpr (Ti::kOwnLater) {
+#pragma unroll
+    for (int t = 0; t < 27; t++) f0s[t * THREADS] = a.f_in[(long long)c_ref27[t] * a.N + idx];
+  }
   double rho0 = 1, U[3] = {0, 0, 0}, T = L::TLat;
   if (active) {  // c0.load (steps.cu:360-363); the populations are in f0s already
     rho0 = a.rho_in[idx];
@@ -786,8 +905,8 @@ __global__ void __launch_bounds__(THREADS, 2) pull_d3q27_tile_kernel(StepArgs<fl
       const unsigned live = __ballot_sync(0xffffffffu, !done);
       if (__popc(live) <= few_lanes<N>()) {
         if (!done) work += 25ull * (5 * 171 + 342);
-        contract_live_lanes<N>(live, sm, sbase, SX, SX * SY, lo, hi, ro, wt, bq, ainv,
-                               sm + NS * SN + 27 * THREADS + (tid >> 5) * 28, acc);
+        contract_live_lanes<N, Ti::ROWS>(live, sm, sbase, SX, SX * SY, lo, hi, ro, wt, bq, ainv,
+                                         sm + Ti::OFF_S + (tid >> 5) * Ti::SERVED, acc);
       } else {
         const bool staggered =
             __all_sync(0xffffffffu, done || (ro[2][1] == wl[2] && ro[2][2] == wl[2] + 1 && ro[2][0] >= wl[2] &&
@@ -863,7 +982,7 @@ __global__ void __launch_bounds__(THREADS, 2) pull_d3q27_tile_kernel(StepArgs<fl
 #pragma unroll
         for (int t = 0; t < 27; t++) acc[t] = 0.f;
       }
-      conv = tile_moments_and_test(a, acc, f0s, THREADS, C, rho0, U, T);
+      conv = tile_moments_and_test<N>(a, acc, f0s, THREADS, C, rho0, U, T);
       if (conv || niter >= a.max_iter) done = true;
     }
   }
@@ -874,7 +993,7 @@ __global__ void __launch_bounds__(THREADS, 2) pull_d3q27_tile_kernel(StepArgs<fl
     finish_node<POND_D3Q27, float>(a, idx, f0, rho0, U, T, niter, conv, ns);
     ns.work = work;
   }
-  if constexpr (kPartials) add_block_partial(ns, reinterpret_cast<BlockPartial*>(a.sums));
+  if constexpr (kPartials) add_block_partial<Ti::WARPS>(ns, reinterpret_cast<BlockPartial*>(a.sums));
   else reduce_and_commit(ns, a.sums);
 }
 

@@ -65,10 +65,12 @@ constexpr int THREADS = 2 * NODES;
 constexpr int OFF_H = NS * SN;
 constexpr int OFF_OWN = 2 * NS * SN;
 constexpr int OFF_X = OFF_OWN + 27 * THREADS;
-constexpr int OFF_S = OFF_X + 2 * (2 * 5 * NODES) + 2 * 2 * NODES;  // 28 floats of scratch per warp
-constexpr int OFF_U = OFF_S + (THREADS / 32) * 28;  // the staged nodes' velocities (T: the pad of their f)
-constexpr size_t SMEM_BYTES = size_t(OFF_U + 3 * SN) * sizeof(float);
-static_assert(OFF_X % 2 == 0, "the float64 exchange slots must be 8-byte aligned");
+// the warps' scratch for served nodes, over the staged nodes' velocities (T: the pad of their f)
+constexpr int OFF_S = OFF_X + 2 * (2 * 5 * NODES) + 2 * 2 * NODES, OFF_U = OFF_S;
+constexpr int ROWS = 3, SERVED = d27::served_floats(ROWS);
+static_assert(3 * SN <= SERVED * (THREADS / 32), "the velocities must fit the scratch");
+constexpr size_t SMEM_BYTES = size_t(OFF_S + SERVED * (THREADS / 32)) * sizeof(float);
+static_assert(OFF_X % 2 == 0 && OFF_S % 4 == 0, "the float64 exchange slots must be 8-byte aligned, the scratch 16-byte");
 static_assert(SMEM_BYTES + 3 * 1024 <= 232448, "the tile must fit one CTA per SM");
 
 __device__ __forceinline__ void pair_barrier(int pair) {
@@ -225,8 +227,8 @@ __global__ void __launch_bounds__(THREADS, 1) pull_d3q27_energy_tile_kernel(Step
       const unsigned live = __ballot_sync(0xffffffffu, !done);
       if (__popc(live) <= few_lanes<N>()) {
         if (!done) work += 25ull * (5 * 171 + 342);
-        contract_live_lanes<N>(live, sd, sbase, SX, SX * SY, lo, hi, ro, wt, bq, ainv,
-                               sm + OFF_S + (tid >> 5) * 28, acc);
+        contract_live_lanes<N, ROWS>(live, sd, sbase, SX, SX * SY, lo, hi, ro, wt, bq, ainv,
+                                     sm + OFF_S + (tid >> 5) * SERVED, acc);
       } else {
         const bool staggered =
             __all_sync(0xffffffffu, done || (ro[2][1] == wl[2] && ro[2][2] == wl[2] + 1 && ro[2][0] >= wl[2] &&
