@@ -273,20 +273,31 @@ __device__ __forceinline__ void copy_node(const float* f, long long N, long long
 }
 
 // moments_and_test for the float32 tiles: the node's previous populations lie
-// in shared memory (`f0`, `stride` floats apart, replaced by acc), and the
-// difference of the populations is taken in float32.
+// in shared memory (`f0`, `stride` floats apart, replaced by acc).  isConv's
+// comparison is float64's: the float32 difference and threshold, each within
+// 3e-7 of the exact one, decide where they lie further apart than 1e-6, and the
+// float64 ones where they do not, or where the threshold is too small for that.
 // Order 3 forms its sums in moments_and_test's order, so that its results stay
 // those of the node-by-node sums to the last bit (128^3: 1 % of the step).
 template <int N>
 __device__ __forceinline__ bool tile_moments_and_test(const StepArgs<float>& a, const float acc[27], float* f0, int stride,
                                                       double C, double& rho0, double U[3], double& T) {
   using L = Lattice<POND_D3Q27>;
-  bool ok = true;
+  const float ta = float(a.tol_abs), tr = float(a.tol_rel);
+  bool ok = true, close = false;
 #pragma unroll
   for (int t = 0; t < 27; t++) {
-    const double nv = acc[t];
-    ok = ok && !(double(fabsf(acc[t] - f0[t * stride])) >= a.tol_abs + a.tol_rel * fabs(nv));
+    const float d = fabsf(acc[t] - f0[t * stride]), thr = fmaf(tr, fabsf(acc[t]), ta);
+    const bool over = d > 1.000001f * thr, under = d < 0.999999f * thr && thr > 1e-30f;
+    ok = ok && !(over && thr > 1e-30f);
+    close = close || !(under || (over && thr > 1e-30f));
   }
+  if (ok && close)
+#pragma unroll 1
+    for (int t = 0; t < 27; t++) {
+      const double nv = acc[t], ov = f0[t * stride];
+      ok = ok && !(fabs(nv - ov) >= a.tol_abs + a.tol_rel * fabs(nv));
+    }
   double m[4] = {0, 0, 0, 0}, rho = 0;
   if constexpr (N == 3) {
 #pragma unroll
