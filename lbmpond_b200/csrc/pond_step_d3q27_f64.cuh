@@ -8,7 +8,8 @@
 // interpolation weights and the transfer R -> target against the R-gauge
 // populations one axis at a time (81 multiply-adds per stencil node, column
 // and row) instead of transforming every stencil node into the target gauge
-// (243).  The two agree to float64 rounding.
+// (243).  While the gauges lie within a factor 2 of the tile's (near_ref) the
+// two agree to 7e-15 of the largest population; other tiles are left out.
 //
 //  * a CTA owns a 10 x 4 x 2 tile, staged with its +-2 halo (14 x 8 x 6 nodes,
 //    161 KB); per node three slices k1 of nine populations, 10 doubles apart, so
@@ -18,14 +19,16 @@
 //    (27 accumulators would not fit a lane in float64: nine do), then, after
 //    the row's exchange through shared memory, target z-class i3 = j for the x
 //    contraction, the moments and the test;
-//  * a warp with a node whose windows leave the halo runs that iteration from
+//  * a warp with a node whose windows leave the halo, or whose iterate
+//    moves far from the tile's gauge, runs that iteration from
 //    global memory: lane 3n + j transforms each stencil node into the target's
 //    z-class j directly, as the one-thread-per-node kernel does for all three.
 //    That takes 2.5-3.5 times the time of the one-thread-per-node kernel (32^3
 //    at c = 1.2: 10.6 against 4.1 ms, 10 nodes per warp instead of 32 and three
 //    loads of each), so it serves nodes that get there while iterating; a tile
 //    with a node that starts near the edge of the halo (|u| + c >= 0.98 on an
-//    axis for N = 4) is flagged and left to that kernel, which follows every
+//    axis for N = 4), or with gauges far from its centre's, is flagged and left to
+//    that kernel, which follows every
 //    launch and returns at once where nothing is flagged (32^3 at c = 0.95 and
 //    |u| up to 0.06: 4.0 ms with a quarter of the rows as the line, against 2.2).
 //
@@ -33,7 +36,7 @@
 // lane and iteration at N = 4 are 2,090 cycles of the SM) and shared-memory
 // bandwidth (17 wavefronts per stencil node, as much), at two warps per
 // scheduler.  48^3 half-uniform blast, cubic, 1e-12 + 1e-10 |v|, 4.8 iterations
-// per node: 1.63 ms per step against 7.02 ms for the one-thread-per-node kernel
+// per node: 1.70 ms per step against 7.02 ms for the one-thread-per-node kernel
 // (three-pass transform of every stencil node, read from L1/L2 per iteration).
 #pragma once
 #include "pond_step_d3q27.cuh"
@@ -58,6 +61,20 @@ struct Smem {
   double ex[WARPS][32 * 9];    // a row's results [3 i2 + i3] of lane (n, k1)
 };
 static_assert(sizeof(Smem) + 4096 <= 232448, "the tile must fit one CTA");
+
+// Whether a gauge (u, c) lies near enough to R that the way through R keeps
+// float64's digits.  A transfer source -> R -> target cancels terms of
+// (|u - u_ref| / c + c ratio)^2 per axis and way; for one node against the
+// direct transfer, both in float64 (random states, relative to the largest
+// population): c within a factor 2 of c_ref and |u - u_ref| up to 1.0 of the
+// smaller c 7e-15 at most (direct: 1e-15); factor 5: 7e-13; factor 10 (a
+// temperature ratio of 100): 2e-11; factor 100: 1e-5.
+constexpr double FAR_C = 2.0, FAR_U = 1.0;
+__device__ __forceinline__ bool near_ref(const double u[3], double c, const double uref[3], double cref, double slack) {
+  const double least = slack * FAR_U * fmin(c, cref);
+  return c <= slack * FAR_C * cref && cref <= slack * FAR_C * c && fabs(u[0] - uref[0]) <= least &&
+         fabs(u[1] - uref[1]) <= least && fabs(u[2] - uref[2]) <= least;
+}
 
 // One stencil node into a column: Z[k2][i3] += sum_k3 c[i3][k3] F[k2][k3] for the
 // z-classes i3 = 0, + (kPlus) and - (kMinus) of this lane's k1
@@ -87,29 +104,6 @@ template <int N> __global__ void __launch_bounds__(THREADS, 1) pull_d3q27_f64_ke
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY, z0 = blockIdx.z * TZ;
   constexpr double kMax = 1.7976931348623157e308;
-
-  // ---- a tile with a node that starts at the edge of the halo or beyond is left to
-  //      the one-thread-per-node kernel launched after this one
-  {
-    const int n = lane % TX, x = x0 + n, y = y0 + warp % TY, z = z0 + warp / TY;
-    const bool here = x < a.nx && y < a.ny && z < a.nz;
-    bool far = false;
-    if (here && lane < TX) {
-      const long long g = x + (long long)a.nx * (y + (long long)a.ny * z);
-      const double c = a.guess ? sqrt(double(a.guess[3 * a.N + g]) * (1.0 / L::TLat))
-                               : sqrt(a.g_in[3 * a.N + g] * (1.0 / L::TLat));
-#pragma unroll
-      for (int ax = 0; ax < 3; ax++) {
-        const double u = fabs(a.guess ? double(a.guess[ax * a.N + g]) : a.g_in[ax * a.N + g]);
-        // the largest |v| whose window stays within two nodes, less what an iterate may add
-        far = far || u + c >= 0.98 * (N == 4 ? 1.0 : N == 2 ? 2.0 : ax == 0 ? 1.5 : 1.0);
-      }
-    }
-    const bool leave = __syncthreads_or(far);
-    if (tid == 0)
-      a.tile_flags[blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z)] = leave;
-    if (leave) return;
-  }
 
   // ---- reference gauge of the CTA: the gauge of the tile's centre node
   //      ((0, 1) if it is not finite or its c is 0)
@@ -154,6 +148,52 @@ template <int N> __global__ void __launch_bounds__(THREADS, 1) pull_d3q27_f64_ke
       asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d + 8 * (10 * (t / 9) + t % 9)),
                    "l"(src + (long long)d27::c_ref27[cx * 9 + cy * 3 + cz] * a.N)
                    : "memory");
+    }
+  }
+  // ---- a tile with a node that starts at the edge of the halo or beyond, or whose
+  //      gauges (halo included) lie further from R than FAR_C and FAR_U, is left to
+  //      the one-thread-per-node kernel launched after this one (looked at while
+  //      the copies are in flight)
+  {
+    const int n = lane % TX, x = x0 + n, y = y0 + warp % TY, z = z0 + warp / TY;
+    const bool here = x < a.nx && y < a.ny && z < a.nz;
+    bool far = false;
+    if (here && lane < TX) {
+      const long long g = x + (long long)a.nx * (y + (long long)a.ny * z);
+      const double c = a.guess ? sqrt(double(a.guess[3 * a.N + g]) * (1.0 / L::TLat))
+                               : sqrt(a.g_in[3 * a.N + g] * (1.0 / L::TLat));
+#pragma unroll
+      for (int ax = 0; ax < 3; ax++) {
+        const double u = fabs(a.guess ? double(a.guess[ax * a.N + g]) : a.g_in[ax * a.N + g]);
+        // the largest |v| whose window stays within two nodes, less what an iterate may add
+        far = far || u + c >= 0.98 * (N == 4 ? 1.0 : N == 2 ? 2.0 : ax == 0 ? 1.5 : 1.0);
+      }
+    }
+    for (int i = tid; i < SN; i += THREADS) {
+      const int hx = i % SX, hy = (i / SX) % SY, hz = i / (SX * SY);
+      bool rv[3];
+      const int gx = resolve_axis(x0 - H + hx, a.nx, a.bc[0], rv[0]);
+      const int gy = resolve_axis(y0 - H + hy, a.ny, a.bc[1], rv[1]);
+      const int gz = resolve_axis(z0 - H + hz, a.nz, a.bc[2], rv[2]);
+      const long long g = gx + (long long)a.nx * (gy + (long long)a.ny * gz);
+      double u[3];
+      bool ok = true;
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        const double v = a.g_in[(long long)k * a.N + g];
+        u[k] = rv[k] ? -v : v;
+        ok = ok && fabs(v) <= kMax;
+      }
+      const double c = sqrt(fabs(a.g_in[3 * a.N + g]) * (1.0 / L::TLat));
+      // nodes without a finite gauge contribute nothing
+      far = far || (ok && c <= kMax && !near_ref(u, c, uref, cref, 1.0));
+    }
+    const bool leave = __syncthreads_or(far);
+    if (tid == 0)
+      a.tile_flags[blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z)] = leave;
+    if (leave) {
+      d27::cp_async_wait_all();
+      return;
     }
   }
   d27::cp_async_wait_all();
@@ -253,7 +293,7 @@ template <int N> __global__ void __launch_bounds__(THREADS, 1) pull_d3q27_f64_ke
     }
     const int zlo = min(rz[0], min(rz[1], rz[2])), zhi = max(rz[0], max(rz[1], rz[2])) + N - 1;
     const int olo = min(ro[0], min(ro[1], ro[2])), ohi = max(ro[0], max(ro[1], ro[2])) + N - 1;
-    const bool inside = zlo >= -H && zhi <= H && olo >= -H && ohi <= H;
+    const bool inside = zlo >= -H && zhi <= H && olo >= -H && ohi <= H && near_ref(U, C, uref, cref, 1.25);
     double acc[3][3];  // [i1][i2] of i3 = j
 #pragma unroll
     for (int i = 0; i < 9; i++) acc[i / 3][i % 3] = 0.0;
