@@ -43,6 +43,7 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <numeric>
 #include <set>
@@ -655,6 +656,7 @@ struct pond_batch {
   std::vector<int> by_pos;       // the problems in bin order
   float* pin = nullptr;          // pinned staging of pond_batch_get_state, from its first call
   cudaEvent_t pin_ev[4] = {nullptr, nullptr, nullptr, nullptr};
+  std::mutex pin_mutex;          // held by the reader that uses them
   std::vector<int> len;
   long long istep = 0;
   cudaGraphExec_t exec = nullptr;
@@ -800,7 +802,26 @@ static void choose_bins(const int32_t* lengths, int P, long long nodes, int sms,
 constexpr long long PAGEABLE_NODES = 200000;
 template <typename Src, typename Dst> static int read_planes(pond_batch* b, int nplanes, Src src, Dst dst) {
   const long long n = b->stride;
-  if (n <= PAGEABLE_NODES) {
+  constexpr long long CHUNK = 1 << 17;  // floats
+  constexpr int BUFS = 4;
+  static_assert(PAGEABLE_NODES > CHUNK, "more than one chunk per plane");
+  std::unique_lock<std::mutex> pinned(b->pin_mutex, std::defer_lock);
+  bool staged = n > PAGEABLE_NODES;
+  if (staged) {
+    pinned.lock();  // one reader at a time: the buffers, the events and the stream are the batch's
+    if (!b->pin && cudaMallocHost(&b->pin, BUFS * CHUNK * sizeof(float)) != cudaSuccess) b->pin = nullptr;
+    staged = b->pin != nullptr;
+    for (int i = 0; i < BUFS && staged; i++)
+      if (!b->pin_ev[i] && cudaEventCreateWithFlags(&b->pin_ev[i], cudaEventDisableTiming) != cudaSuccess) {
+        b->pin_ev[i] = nullptr;
+        staged = false;
+      }
+    if (!staged) {  // no pinned memory or event to be had: the plain copies need neither
+      cudaGetLastError();
+      pinned.unlock();
+    }
+  }
+  if (!staged) {
     std::vector<float> tmp(n);
     for (int i = 0; i < nplanes; i++) {
       const cudaError_t e = cudaMemcpy(tmp.data(), src(i), n * sizeof(float), cudaMemcpyDeviceToHost);
@@ -811,18 +832,9 @@ template <typename Src, typename Dst> static int read_planes(pond_batch* b, int 
     }
     return POND_OK;
   }
-  constexpr long long CHUNK = 1 << 17;  // floats
-  constexpr int BUFS = 4;
-  if (!b->pin) {
-    const cudaError_t e = cudaMallocHost(&b->pin, BUFS * CHUNK * sizeof(float));
-    if (e != cudaSuccess) return cuda_fail(e, "pond_batch_get_state staging");
-    for (int i = 0; i < BUFS; i++)
-      if (cudaEventCreateWithFlags(&b->pin_ev[i], cudaEventDisableTiming) != cudaSuccess)
-        return cuda_fail(cudaGetLastError(), "pond_batch_get_state events");
-  }
   const long long per = (n + CHUNK - 1) / CHUNK, chunks = per * nplanes;
   const int hw = (int)std::thread::hardware_concurrency();
-  const int workers = chunks <= nplanes ? 1 : std::max(1, std::min(8, hw));
+  const int workers = std::max(1, std::min(8, hw));
   std::atomic<long long> issued{0};
   std::atomic<bool> stop{false};
   std::vector<std::atomic<int>> done(chunks);
@@ -891,6 +903,7 @@ template <typename Src, typename Dst> static int read_planes(pond_batch* b, int 
   if (e != cudaSuccess) stop.store(true);
   for (auto& t : pool) t.join();
   if (e == cudaSuccess && stop.load()) e = cudaErrorUnknown;
+  if (e != cudaSuccess) cudaStreamSynchronize(b->stream);  // no copy still fills the buffers when the next reader takes them
   return e == cudaSuccess ? POND_OK : cuda_fail(e, "pond_batch_get_state");
 }
 
@@ -1071,6 +1084,8 @@ int pond_batch_get_state(pond_batch* b, double* f, double* rho, double* u, doubl
                               [&](int i) { return planes[i].dst; });
   } catch (const std::bad_alloc&) {
     return set_error(POND_ERR_NOMEM, "pond_batch_get_state: host memory");
+  } catch (const std::exception& x) {
+    return set_error(POND_ERR_STATE, "pond_batch_get_state: %s", x.what());
   }
 }
 
