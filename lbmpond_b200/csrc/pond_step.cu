@@ -204,7 +204,8 @@ static int gap2_ctas(int nx) { return (nx + 127) / 128 < 148 * 6 ? (nx + 127) / 
 
 // Launch a step kernel that may start while the step before it on the stream
 // runs its last CTAs; it waits in the kernel for that step to complete
-// (cudaGridDependencySynchronize).  Hides the launch of every step but the
+// (cudaGridDependencySynchronize), and reads what that step writes by plain loads
+// only.  Hides the launch of every step but the
 // first: 1000 nodes of D1Q5 9.2 us per step instead of 10.3.
 template <typename R>
 static cudaError_t launch_early(void (*kern)(StepArgs<R>), dim3 grid, dim3 block, size_t smem, cudaStream_t s,

@@ -24,16 +24,19 @@ constexpr int THREADS = 32 * WARPS;
 constexpr int LANES = 6;  // per population
 
 // population k of grid node p (boundaries resolved) in the gauge (Uc, 1/invC):
-// row k of the 5-point basis of the node's speeds, non-finite terms dropped
+// row k of the 5-point basis of the node's speeds, non-finite terms dropped.
+// Plain loads: the kernel is resident while the step before still writes its
+// inputs, and the read-only path (__ldg) is for data that nothing writes as
+// long as the kernel lives.
 template <typename R>
 __device__ __forceinline__ R transfer_row(const StepArgs<R>& a, int p, int k, R Uc, R invC) {
   using L = Lattice<POND_D1Q5>;
   bool rv;
   const long long n = resolve_axis(p, a.nx, a.bc[0], rv);
-  const R T = __ldg(&a.g_in[3 * a.N + n]), u = __ldg(&a.g_in[n]);
+  const R T = a.g_in[3 * a.N + n], u = a.g_in[n];
   R f[5];
 #pragma unroll
-  for (int b = 0; b < 5; b++) f[b] = finite_or_zero_f(__ldg(&a.f_in[b * a.N + n]));
+  for (int b = 0; b < 5; b++) f[b] = finite_or_zero_f(a.f_in[b * a.N + n]);
   const R c = copysign(sqrt(fabs(T) * R(1.0 / L::TLat)), T);
   const R s = ((rv ? -u : u) - Uc) * invC, r = (rv ? -c : c) * invC;
   constexpr double e1s = EC1 * EC1, e2s = EC2 * EC2;

@@ -965,10 +965,10 @@ __global__ void __launch_bounds__(Tile<N>::THREADS, Tile<N>::CTAS) pull_d3q27_ti
             const bool ok = fabsf(un[0]) <= 3.0e38f && fabsf(un[1]) <= 3.0e38f && fabsf(un[2]) <= 3.0e38f &&
                             fabsf(Tn) <= 3.0e38f;
             const float cn = copysignf(sqrtf(fabsf(Tn) * (float)(1.0 / L::TLat)), Tn);
-            float v[27];
+            float v[27];  // plain loads: f_in may have been written while this kernel was resident
 #pragma unroll
             for (int t = 0; t < 27; t++)
-              v[t] = ok ? finite_or_zero_f(__ldg(&a.f_in[(long long)c_ref27[t] * a.N + g])) : 0.f;
+              v[t] = ok ? finite_or_zero_f(a.f_in[(long long)c_ref27[t] * a.N + g]) : 0.f;
             float sq[3], rq[3];
 #pragma unroll
             for (int k = 0; k < 3; k++) {
