@@ -326,7 +326,7 @@ int pond_predict(pond_ctx* ctx, float* guess);
    that owns all device memory through its own pool or a budget fixed at
    start-up, or that must not stall on an allocation inside its time loop.
    It calls no cudaMalloc, cudaFree or allocating library routine.  Its only
-   scratch, an array of partial-sum records, lives in a fixed
+   scratch, one partial-sum record per step CTA, lives in a fixed
    POND_NOALLOC_SCRATCH_BYTES array in the library's device memory, which
    every GPU that loads the library holds until the process exits.  Grids of
    more than 65536 blocks of 32x4x2 nodes (256^3 nodes) are rejected with

@@ -7,8 +7,8 @@
 // loop, or a runtime that hands out device memory only through its own
 // allocator.  The context API allocates its double buffers and reduction
 // slots in pond_create; this entry point takes the caller's input and output
-// buffers and keeps its only scratch -- an array of partial-sum records, each
-// shared by at most a few CTAs of the step kernel -- in a fixed array in this file's device memory.
+// buffers and keeps its only scratch -- one partial-sum record per CTA of the
+// step kernel -- in a fixed array in this file's device memory.
 //
 // The scratch array is a file-scope __device__ variable: every GPU that
 // loads the library holds POND_NOALLOC_SCRATCH_BYTES of it until the process
@@ -29,7 +29,7 @@ namespace pond {
 namespace noalloc {
 
 constexpr int kMaxBlocks = 65536;  // largest grid accepted, in blocks of 32x4x2 nodes (256^3 nodes)
-constexpr size_t kScratchBytes = size_t(d27::PARTIALS) * sizeof(d27::BlockPartial);
+constexpr size_t kScratchBytes = size_t(kMaxBlocks) * sizeof(d27::BlockPartial);  // a record per CTA of the step
 static_assert(kScratchBytes == POND_NOALLOC_SCRATCH_BYTES, "pond.h states the scratch size");
 
 static __device__ __align__(256) unsigned char g_partials[kScratchBytes];
@@ -38,11 +38,8 @@ constexpr int kMaxDevices = 64;
 static std::mutex g_setup_mutex;
 static void* g_partials_addr[kMaxDevices] = {};
 
-// Sum the records in a fixed order and write the step's diagnostics to the
-// caller's buffer.  A record holds the sums of one or two CTAs up to 256^3
-// nodes in grids of three or more z planes, and two terms add to the same
-// value in either order, so the result does not depend on CTA scheduling
-// there; flatter grids near the size limit share a record among up to four.
+// Sum the per-CTA records in a fixed order (the result does not depend on
+// CTA scheduling) and write the step's diagnostics to the caller's buffer.
 __global__ void __launch_bounds__(256) reduce_partials_kernel(const d27::BlockPartial* part, int nrec,
                                                               long long N, pond_diag* out) {
   __shared__ double sd[6][256];
@@ -100,20 +97,17 @@ static bool any_overlap(long long N, const float* fi, const float* ri, const flo
   return false;
 }
 
-template <int N> static dim3 grid(const StepArgs<float>& a) {
+// The step on at most kMaxBlocks CTAs, one record each; returns their number.
+template <int N> static int launch(const StepArgs<float>& a, d27::BlockPartial* records, cudaStream_t s) {
   using Ti = d27::Tile<N>;
-  return dim3((a.nx + Ti::TX - 1) / Ti::TX, (a.ny + Ti::TY - 1) / Ti::TY, (a.nz + Ti::TZ - 1) / Ti::TZ);
-}
-template <int N> static long long ctas(const StepArgs<float>& a) {
-  const dim3 g = grid<N>(a);
-  return (long long)g.x * g.y * g.z;
-}
-template <int N> static void launch(const StepArgs<float>& a, cudaStream_t s) {
-  using Ti = d27::Tile<N>;
-  d27::pull_d3q27_tile_kernel<N, true><<<grid<N>(a), Ti::THREADS, Ti::SMEM_BYTES, s>>>(a);
+  const int nx = (a.nx + Ti::TX - 1) / Ti::TX, ny = (a.ny + Ti::TY - 1) / Ti::TY, nz = (a.nz + Ti::TZ - 1) / Ti::TZ;
+  const int tiles = nx * ny * nz;  // at most four per block of 32x4x2 nodes
+  const int ctas = tiles < kMaxBlocks ? tiles : kMaxBlocks;
+  d27::pull_d3q27_records_kernel<N><<<ctas, Ti::THREADS, Ti::SMEM_BYTES, s>>>(a, nx, ny, tiles, records);
+  return ctas;
 }
 template <int N> static cudaError_t opt_in() {
-  return cudaFuncSetAttribute(d27::pull_d3q27_tile_kernel<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  return cudaFuncSetAttribute(d27::pull_d3q27_records_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)d27::Tile<N>::SMEM_BYTES);
 }
 
@@ -178,7 +172,7 @@ extern "C" int pond_step_noalloc(const pond_params* p, const float* f_in, const 
   a.f_out = f_out; a.rho_out = rho_out; a.g_out = g_out;
   a.guess = nullptr;
   a.niter_out = nullptr;
-  a.sums = reinterpret_cast<StepSums*>(scratch);  // the partial records
+  a.sums = nullptr;  // the records instead
   a.nx = (int)p->Nx; a.ny = (int)p->Ny; a.nz = (int)p->Nz;
   a.N = N;
   for (int k = 0; k < 3; k++) a.bc[k] = p->bc[k];
@@ -189,19 +183,13 @@ extern "C" int pond_step_noalloc(const pond_params* p, const float* f_in, const 
   const double PI = 3.14159265358979323846;
   a.kdx = 0.5 / (8 * PI * PI * PI) * (2 * PI / p->Nx) * (2 * PI / p->Ny) * (2 * PI / p->Nz);
   cudaStream_t s = (cudaStream_t)stream;
-  const long long ctas = p->interp == POND_LAGR2   ? noalloc::ctas<2>(a)
-                         : p->interp == POND_LAGR3 ? noalloc::ctas<3>(a)
-                                                   : noalloc::ctas<4>(a);
-  const int nrec = (int)(ctas < d27::PARTIALS ? ctas : d27::PARTIALS);
-  cudaError_t e = cudaMemsetAsync(scratch, 0, (size_t)nrec * sizeof(d27::BlockPartial), s);
-  if (e != cudaSuccess) return cuda_fail(e, "pond_step_noalloc scratch reset");
-  if (p->interp == POND_LAGR2) noalloc::launch<2>(a, s);
-  else if (p->interp == POND_LAGR3) noalloc::launch<3>(a, s);
-  else noalloc::launch<4>(a, s);
-  e = cudaGetLastError();
+  auto* records = reinterpret_cast<d27::BlockPartial*>(scratch);
+  const int nrec = p->interp == POND_LAGR2   ? noalloc::launch<2>(a, records, s)
+                   : p->interp == POND_LAGR3 ? noalloc::launch<3>(a, records, s)
+                                             : noalloc::launch<4>(a, records, s);
+  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "pond_step_noalloc step launch");
-  noalloc::reduce_partials_kernel<<<1, 256, 0, s>>>(reinterpret_cast<const d27::BlockPartial*>(scratch),
-                                                      nrec, N, diag_out);
+  noalloc::reduce_partials_kernel<<<1, 256, 0, s>>>(records, nrec, N, diag_out);
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "pond_step_noalloc reduction launch");
   return POND_OK;

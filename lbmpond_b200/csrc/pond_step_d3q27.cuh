@@ -698,11 +698,8 @@ __device__ __forceinline__ void contract_live_lanes(unsigned live, const float* 
 // are within 0.7 % of each other from 32^3 to 256^3, 8 lanes 0.5-4 % slower.
 template <int N> __host__ __device__ constexpr int few_lanes() { return N == 4 ? 5 : N == 3 ? 3 : 2; }
 
-// Partial record of the step sums, updated instead of the context's sums
-// when the kernel runs without a context (kPartials = true; a.sums then
-// points at an array of PARTIALS zeroed records, CTA b adding to record
-// b % PARTIALS).
-constexpr int PARTIALS = 65536;
+// Record of a CTA's step sums, written instead of the context's sums when the
+// kernel runs without a context.
 struct BlockPartial {
   double mass, mom[3], enrg, k;
   unsigned long long niter_sum, nonconv, work;
@@ -710,7 +707,8 @@ struct BlockPartial {
   int pad;
 };
 
-template <int WARPS> __device__ __forceinline__ void add_block_partial(NodeSums s, BlockPartial* out) {
+// Add the CTA's sums to `sum` (in shared memory), in a fixed order.
+template <int WARPS> __device__ __forceinline__ void add_block_partial(NodeSums s, BlockPartial& sum) {
   __shared__ double pd[6][WARPS];
   __shared__ unsigned long long pu[3][WARPS];
   __shared__ int pm[WARPS];
@@ -732,28 +730,21 @@ template <int WARPS> __device__ __forceinline__ void add_block_partial(NodeSums 
   }
   __syncthreads();
   if (tid == 0) {
-    BlockPartial b = {};
+    BlockPartial b = sum;
     for (int w = 0; w < WARPS; w++) {
       b.mass += pd[0][w]; b.mom[0] += pd[1][w]; b.mom[1] += pd[2][w]; b.mom[2] += pd[3][w];
       b.enrg += pd[4][w]; b.k += pd[5][w];
       b.niter_sum += pu[0][w]; b.nonconv += pu[1][w]; b.work += pu[2][w];
       b.niter_max = max(b.niter_max, pm[w]);
     }
-    const unsigned long long cta =
-        blockIdx.x + (unsigned long long)gridDim.x * (blockIdx.y + (unsigned long long)gridDim.y * blockIdx.z);
-    BlockPartial* o = out + cta % PARTIALS;
-    atomicAdd(&o->mass, b.mass);
-    for (int q = 0; q < 3; q++) atomicAdd(&o->mom[q], b.mom[q]);
-    atomicAdd(&o->enrg, b.enrg);
-    atomicAdd(&o->k, b.k);
-    atomicAdd(&o->niter_sum, b.niter_sum);
-    if (b.nonconv) atomicAdd(&o->nonconv, b.nonconv);
-    atomicMax(&o->niter_max, b.niter_max);
+    sum = b;
   }
 }
 
-template <int N, bool kPartials = false>
-__global__ void __launch_bounds__(Tile<N>::THREADS, Tile<N>::CTAS) pull_d3q27_tile_kernel(StepArgs<float> a) {
+// The step of the tile whose first node is (x0, y0, z0), by one CTA; `ns`
+// gains this thread's share of the sums.
+template <int N>
+__device__ __forceinline__ void step_tile(const StepArgs<float>& a, const int x0, const int y0, const int z0, NodeSums& ns) {
   using L = Lattice<POND_D3Q27>;
   using Ti = Tile<N>;
   constexpr int SX = Ti::SX, SY = Ti::SY, SN = Ti::SN, THREADS = Ti::THREADS;
@@ -761,11 +752,6 @@ __global__ void __launch_bounds__(Tile<N>::THREADS, Tile<N>::CTAS) pull_d3q27_ti
   const int tid = threadIdx.x;
   float* own = sm + Ti::OFF_OWN;
   float* su = sm + Ti::OFF_U;
-  const int x0 = blockIdx.x * Ti::TX, y0 = blockIdx.y * Ti::TY, z0 = blockIdx.z * Ti::TZ;
-  // launched while the step before still runs (launch_early): let the next one
-  // come, then wait for the step before to be complete and visible
-  cudaTriggerProgrammaticLaunchCompletion();
-  cudaGridDependencySynchronize();
 
   // ---- stage: each thread copies whole staged nodes (27 populations, the
   // mirror reversing classes, and the gauge) with asynchronous copies, waits
@@ -845,7 +831,6 @@ __global__ void __launch_bounds__(Tile<N>::THREADS, Tile<N>::CTAS) pull_d3q27_ti
   const int lx = Ti::lx(tid), ly = Ti::ly(tid), lz = Ti::lz(tid);
   const int x = x0 + lx, y = y0 + ly, z = z0 + lz;
   const bool active = x < a.nx && y < a.ny && z < a.nz;
-  NodeSums ns = {0, 0, 0, 0, 0, 0, 0ull, 0ull, 0ull, 0};
   const long long idx = active ? x + (long long)a.nx * (y + (long long)a.ny * z) : 0;
   // the node's current populations live in shared memory between iterations,
   // which keeps them out of the loop's registers
@@ -1001,11 +986,41 @@ __global__ void __launch_bounds__(Tile<N>::THREADS, Tile<N>::CTAS) pull_d3q27_ti
     float f0[27];
 #pragma unroll
     for (int t = 0; t < 27; t++) f0[t] = f0s[t * THREADS];
-    finish_node<POND_D3Q27, float>(a, idx, f0, rho0, U, T, niter, conv, ns);
-    ns.work = work;
+    NodeSums one;
+    finish_node<POND_D3Q27, float>(a, idx, f0, rho0, U, T, niter, conv, one);
+    ns.mass += one.mass; ns.m0 += one.m0; ns.m1 += one.m1; ns.m2 += one.m2; ns.enrg += one.enrg; ns.k += one.k;
+    ns.niter += one.niter; ns.nonconv += one.nonconv; ns.work += work; ns.nmax = max(ns.nmax, one.nmax);
   }
-  if constexpr (kPartials) add_block_partial<Ti::WARPS>(ns, reinterpret_cast<BlockPartial*>(a.sums));
-  else reduce_and_commit(ns, a.sums);
+}
+
+template <int N> __global__ void __launch_bounds__(Tile<N>::THREADS, Tile<N>::CTAS) pull_d3q27_tile_kernel(StepArgs<float> a) {
+  NodeSums ns = {0, 0, 0, 0, 0, 0, 0ull, 0ull, 0ull, 0};
+  // launched while the step before still runs (launch_early): let the next one
+  // come, then wait for the step before to be complete and visible
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
+  step_tile<N>(a, blockIdx.x * Tile<N>::TX, blockIdx.y * Tile<N>::TY, blockIdx.z * Tile<N>::TZ, ns);
+  reduce_and_commit(ns, a.sums);
+}
+
+// The step without a context: of the nx x ny x .. = `tiles` tiles CTA b takes b,
+// b + gridDim.x, .. in turn and writes record b, so that the sums come out the
+// same however the CTAs are scheduled.  (Order 3 has a CTA per tile: an accepted
+// grid has no more of its tiles than records.)
+template <int N>
+__global__ void __launch_bounds__(Tile<N>::THREADS, Tile<N>::CTAS)
+    pull_d3q27_records_kernel(StepArgs<float> a, int nx, int ny, int tiles, BlockPartial* records) {
+  __shared__ BlockPartial sum;
+  if (threadIdx.x == 0) sum = {};
+  int t = blockIdx.x;
+#pragma unroll 1
+  do {
+    NodeSums ns = {0, 0, 0, 0, 0, 0, 0ull, 0ull, 0ull, 0};
+    step_tile<N>(a, t % nx * Tile<N>::TX, t / nx % ny * Tile<N>::TY, t / nx / ny * Tile<N>::TZ, ns);
+    add_block_partial<Tile<N>::WARPS>(ns, sum);  // its barrier ends the tile's use of shared memory
+    t += gridDim.x;
+  } while (N != 3 && t < tiles);
+  if (threadIdx.x == 0) records[blockIdx.x] = sum;
 }
 
 }  // namespace d27
