@@ -206,7 +206,9 @@ int pond_copy_state(pond_ctx* dst, pond_ctx* src);
 /* work of the last step, summed over nodes and iterations (the count behind
    the compute roofline): for the D3Q27 float32 kernel the floating-point
    operations of its basis contractions (a multiply-add counts 2), for the
-   other kernels the stencil nodes transformed */
+   other kernels the stencil nodes of the scheme, each position that one of the
+   node's windows holds once (POND_TVD and POND_WENO5: each from the first to the
+   last; POND_GAP2: two per population), however the kernel transfers them */
 int pond_last_step_work(pond_ctx* ctx, int64_t* work);
 
 /* ---- one-dimensional mesh: node mask, AMR, node positions -------------

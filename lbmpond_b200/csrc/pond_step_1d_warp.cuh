@@ -54,6 +54,18 @@ __device__ __forceinline__ R transfer_row(const StepArgs<R>& a, int p, int k, R 
   return g;
 }
 
+// positions in the union of the warp's windows [org, org + N), as
+// window_positions counts them for the thread-per-node kernels
+template <int N> __device__ __forceinline__ int union_positions(int org) {
+  const int lo = __reduce_min_sync(0xffffffffu, org);
+  if (__reduce_max_sync(0xffffffffu, org) - lo <= 32 - N)
+    return __popc(__reduce_or_sync(0xffffffffu, ((1u << N) - 1u) << (org - lo)));
+  int start[5];
+#pragma unroll
+  for (int k = 0; k < 5; k++) start[k] = __shfl_sync(0xffffffffu, org, LANES * k);
+  return window_positions<N, 5>(start);
+}
+
 template <int SCHEME, typename R> __global__ void __launch_bounds__(THREADS) pull_1d_warp_kernel(StepArgs<R> a) {
   using L = Lattice<POND_D1Q5>;
   constexpr int N = SCHEME == POND_TVD ? 4 : SCHEME == POND_WENO5 ? 5 : SCHEME;  // window nodes
@@ -87,6 +99,7 @@ template <int SCHEME, typename R> __global__ void __launch_bounds__(THREADS) pul
         const double mult = m == 0 ? -2.0 : m == 1 ? -1.0 : m == 2 ? 0.0 : 1.0;
         const double crd = double(x) + v * mult;
         const int org = window_origin<4>(crd, 0);
+        ns.work += (unsigned long long)(__reduce_max_sync(0xffffffffu, org) + 4 - __reduce_min_sync(0xffffffffu, org));
         R w[4];
         lagr_weights<4, R>(crd - double(org), w);
         // the union of the four windows: consecutive nodes while |v| < 1
@@ -113,6 +126,7 @@ template <int SCHEME, typename R> __global__ void __launch_bounds__(THREADS) pul
         fk = R(tvd_combine(Fm[0], Fm[1], Fm[2], Fm[3], v));
       } else if constexpr (SCHEME == POND_WENO5) {
         const int base = (int)(floor(held_coordinate(double(x) - v) + 0.5) - 2);
+        ns.work += (unsigned long long)(__reduce_max_sync(0xffffffffu, base) + 5 - __reduce_min_sync(0xffffffffu, base));
         const R g = transfer_row<R>(a, base + min(e, 4), k, Uc, invC);
         double u[5];
 #pragma unroll
@@ -121,6 +135,7 @@ template <int SCHEME, typename R> __global__ void __launch_bounds__(THREADS) pul
       } else {
         const double crd = double(x) - v;
         const int org = window_origin<N>(crd, 0);
+        ns.work += union_positions<N>(org);
         const double sh = crd - double(org);
         R w[N];
         if (N == 2) {  // LinPol
@@ -134,7 +149,6 @@ template <int SCHEME, typename R> __global__ void __launch_bounds__(THREADS) pul
 #pragma unroll
         for (int j = 0; j < N; j++) fk += w[j] * __shfl_sync(0xffffffffu, g, LANES * k + j);
       }
-      ns.work += N;
       R fn[5];
 #pragma unroll
       for (int q = 0; q < 5; q++) fn[q] = __shfl_sync(0xffffffffu, fk, LANES * q);

@@ -226,7 +226,10 @@ __global__ void __launch_bounds__(THREADS, 1) pull_d3q27_energy_tile_kernel(Step
       }
       const unsigned live = __ballot_sync(0xffffffffu, !done);
       if (__popc(live) <= few_lanes<N>()) {
-        if (!done) work += 25ull * (5 * 171 + 342);
+        if (!done) {  // the node's own windows
+          const unsigned long long ex = hi[0] - lo[0] + 1, ey = hi[1] - lo[1] + 1, ez = hi[2] - lo[2] + 1;
+          work += ex * ey * ez * 171 + ex * ey * 171 + ex * 171;
+        }
         contract_live_lanes<N, ROWS>(live, sd, sbase, SX, SX * SY, lo, hi, ro, wt, bq, ainv,
                                      sm + OFF_S + (tid >> 5) * SERVED, acc);
       } else {

@@ -323,7 +323,15 @@ template <int N> __global__ void __launch_bounds__(THREADS, 1) pull_d3q27_f64_ke
                 wyh = __reduce_max_sync(0xffffffffu, done || !other ? -H : ohi);
       const int wxl = __reduce_min_sync(0xffffffffu, done || other ? H : olo),
                 wxh = __reduce_max_sync(0xffffffffu, done || other ? -H : ohi);
-      if (!done) work += (unsigned long long)(wxh - wxl + 1) * (wyh - wyl + 1) * (wzh - wzl + 1);
+      // the stencil nodes of the node's own windows (x in lane 3n + 1, y in lane 3n)
+      unsigned oz = 0, oo = 0;
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        oz |= ((1u << N) - 1u) << ((rz[c] + H) & 31);
+        oo |= ((1u << N) - 1u) << ((ro[c] + H) & 31);
+      }
+      const int positions = __popc(__shfl_sync(0xffffffffu, oo, 3 * n)) * __popc(__shfl_sync(0xffffffffu, oo, 3 * n + 1)) * __popc(oz);
+      if (!done) work += (unsigned long long)positions;
       // the usual z windows: every lane's + class starts at wzl, its - class one later, wzh = wzl + N;
       // the first offset then has no - class and the last one no + class
       const bool staggered = __all_sync(0xffffffffu, done || (rz[1] == wzl && rz[2] == wzl + 1 && rz[0] >= wzl &&
