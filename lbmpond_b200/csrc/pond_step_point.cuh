@@ -43,10 +43,12 @@ template <int N, typename R> __device__ __forceinline__ void lagr_weights(double
 // Window origin of propagate<N> along one axis (steps.cu:996-997: even N use
 // floor(c)-N/2+1; odd N use floor(c+0.5)-(N-1)/2 in x and floor(c)-(N-1)/2
 // in y and z).
-// A coordinate beyond +-2^29 (a diverged gauge) is held there, so origins,
-// offsets and the positions built from them stay inside int; a NaN stays NaN.
+// A coordinate beyond +-2^29 (a diverged gauge) is held there and a NaN taken as
+// 0, so origins, offsets and the positions built from them stay inside int and
+// the walks over them end (a NaN converts to INT_MIN, whose offset from a node at
+// position N wraps to windows that end at INT_MAX); a NaN's weights stay NaN.
 template <int N> __device__ __forceinline__ int window_origin(double c, int axis) {
-  if (fabs(c) > 536870912.0) c = copysign(536870912.0, c);
+  if (!(fabs(c) <= 536870912.0)) c = c != c ? 0.0 : copysign(536870912.0, c);
   if (N % 2 == 0) return (int)(floor(c) - N / 2 + 1);
   if (axis == 0) return (int)(floor(c + 0.5) - (N - 1) / 2);
   return (int)(floor(c) - (N - 1) / 2);
