@@ -181,8 +181,8 @@ __global__ void __launch_bounds__(THREADS, 1) pull_d3q125_weno_tile_kernel(StepA
   {
     const bool part = lane < 30;
     const int n = part ? lane / 5 : 5, j = part ? lane % 5 : lane - 30;
-    // the exchange (30 lanes x 28 floats) uses this warp's table space
-    static_assert(sizeof(WarpTables) >= 32 * 24 * sizeof(float), "room for the transfer's exchange");
+    // the exchange (20 floats of each of the 32 lanes) uses this warp's table space
+    static_assert(sizeof(WarpTables) >= 32 * 20 * sizeof(float), "room for the transfer's exchange");
     float* ex = reinterpret_cast<float*>(&sm.wt[warp]);
     const float icref = 1.f / cref;
 #pragma unroll 1
