@@ -9,6 +9,7 @@ struct pond_ctx {
   int Q = 0;
   long long N = 0;
   size_t elem = 4;           // bytes per stored value (float or double)
+  int sms = 0;               // multiprocessors of the device
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // double-buffered SoA state: f[Q][N], rho[N], g[4][N]; cur is the latest

@@ -27,6 +27,8 @@ int ctx_alloc(pond_ctx* c) {
   if (e != cudaSuccess) return cuda_fail(e, "cudaStreamCreate");
   if ((e = cudaEventCreate(&c->ev0)) != cudaSuccess) return cuda_fail(e, "cudaEventCreate");
   if ((e = cudaEventCreate(&c->ev1)) != cudaSuccess) return cuda_fail(e, "cudaEventCreate");
+  if ((e = cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->p.device)) != cudaSuccess)
+    return cuda_fail(e, "cudaDeviceGetAttribute");
   const size_t N = (size_t)c->N;
   for (int b = 0; b < 2; b++) {
     if (cudaMalloc(&c->f[b], (size_t)c->Q * N * c->elem) != cudaSuccess ||
@@ -200,7 +202,7 @@ template <int LAT, int N, typename R> static void launch_point(const StepArgs<R>
 // most of it the CTAs' additions to the step's sums).  NONUNIFORM3 keeps a CTA
 // per window: its node setup leaves fewer warps to hide the loop's barriers
 // (4M nodes: 0.51 ms, 0.73 ms looped).
-static int gap2_ctas(int nx) { return (nx + 127) / 128 < 148 * 6 ? (nx + 127) / 128 : 148 * 6; }
+static int gap2_ctas(int nx, int sms) { return (nx + 127) / 128 < sms * 6 ? (nx + 127) / 128 : sms * 6; }
 
 // Launch a step kernel that may start while the step before it on the stream
 // runs its last CTAs; it waits in the kernel for that step to complete
@@ -402,7 +404,7 @@ template <typename R> static int launch_typed(pond_ctx* c, const void* const* in
           pull_1d_scheme_kernel<POND_WENO5, R><<<(a.nx + 127) / 128, 128, 0, s>>>(a);
           break;
         case POND_GAP2:
-          pull_1d_mesh_kernel<POND_GAP2, R><<<gap2_ctas(a.nx), 128, 0, s>>>(a);
+          pull_1d_mesh_kernel<POND_GAP2, R><<<gap2_ctas(a.nx, c->sms), 128, 0, s>>>(a);
           break;
         case POND_NONUNIFORM3:
           pull_1d_mesh_kernel<POND_NONUNIFORM3, R><<<(a.nx + 127) / 128, 128, 0, s>>>(a);
