@@ -293,7 +293,7 @@ __device__ __forceinline__ bool tile_moments_and_test(const StepArgs<float>& a, 
     close = close || !(under || (over && thr > 1e-30f));
   }
   if (ok && close)
-#pragma unroll 1
+#pragma unroll
     for (int t = 0; t < 27; t++) {
       const double nv = acc[t], ov = f0[t * stride];
       ok = ok && !(fabs(nv - ov) >= a.tol_abs + a.tol_rel * fabs(nv));
