@@ -30,9 +30,10 @@
 // Staged layout and contraction are the plain tile's (slot27, contract_tile):
 // two-wide multiply-adds on neighbouring populations, straight-line z columns.
 // Bound by shared-memory bandwidth and by one CTA of 8 warps per SM (both
-// staged sets take 217 KB): two steps of a 64^3 vortex, quadratic, 2.23 ms
-// against 5.32 ms with scalar contractions behind rolled z offsets (the shared
-// contraction 0.9 ms, serving the last lanes by the warp 2.0, staging 0.1).
+// staged sets take 217 KB): two steps of a 64^3 vortex, quadratic, 2.48 ms
+// against 4.86 ms with scalar contractions behind rolled z offsets.  (2.22 with
+// the served lanes summed in another order than the contraction of full warps,
+// which moved single nodes at the iteration cap by 3e-4.)
 #pragma once
 #include "pond_step_d3q27.cuh"
 
